@@ -16,8 +16,7 @@ constexpr int TLD = NB + 1;
 // column-major with leading dimension PLD.  FP32: 68, a multiple of 16
 // bytes, so a thread reads four rows of a column, or two rows of a column,
 // as one vector, and the eight columns a warp reads at once sit in
-// distinct banks.  FP64: the odd stride TLD (scalar loads).  The tile
-// factorization keeps TLD and hands Linv over in this layout.
+// distinct banks.  FP64: the odd stride TLD (scalar loads).
 template <typename T>
 __host__ __device__ constexpr int pld() {
   return sizeof(T) == 4 ? NB + 4 : TLD;
@@ -75,29 +74,44 @@ __device__ __forceinline__ float recip_rn(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double recip_rn(double x) { return __drcp_rn(x); }
 
 // The pivot reciprocal of the tile factorization, on the pivot chain.
-// FP32: the hardware approximation (rcp.approx.f32) refined by one
+// FP32: the hardware approximation (rcp.approx.ftz.f32) refined by one
 // Newton-Raphson step in its FMA form, e = 1 - x r0, r = r0 + r0 e
 // (Markstein, "IA-64 and Elementary Functions", 2000): the refined value
 // is within one ulp of the correctly rounded reciprocal and nearly always
-// equal to it (snu_check_pivot_reciprocal measures both on the GPU), at
-// about half the latency of the correctly rounded one.  FP64: the correctly
-// rounded reciprocal.  A zero or infinite FP32 pivot gives NaN here; the
-// tile factorization flags such pivots either way.
-__device__ __forceinline__ float pivot_recip(float x) {
+// equal to it (snu_check_pivot_reciprocal measures both on the GPU).  The
+// .ftz form is one instruction, where the form that keeps subnormals added
+// 55 cycles to every pivot; pivots whose value or reciprocal it could flush
+// (outside [2^-120, 2^120]) take the same steps on a scaled pivot, in
+// pivot_recip only.  FP64: the correctly rounded reciprocal.  A zero or
+// infinite FP32 pivot gives NaN here; the tile factorization flags such
+// pivots either way.
+__device__ __forceinline__ float pivot_recip_fast(float x) {
   float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   const float e = fmaf(-x, r, 1.f);
   return fmaf(r, e, r);
 }
+__device__ __forceinline__ double pivot_recip_fast(double x) { return __drcp_rn(x); }
+__device__ __forceinline__ float pivot_recip(float x) {
+  const float a = fabsf(x);
+  const float sc = a < 0x1p-120f ? 0x1p64f : a > 0x1p120f ? 0x1p-64f : 1.f;
+  return pivot_recip_fast(x * sc) * sc;
+}
 __device__ __forceinline__ double pivot_recip(double x) { return __drcp_rn(x); }
+// The pivots pivot_recip_fast serves: lo <= |x| <= hi.
+template <typename T>
+__device__ __forceinline__ T pivot_lo() { return sizeof(T) == 4 ? (T)0x1p-120 : (T)4.9406564584124654e-324; }
+template <typename T>
+__device__ __forceinline__ T pivot_hi() { return sizeof(T) == 4 ? (T)0x1p120 : (T)1.7976931348623157e308; }
 
-// Dynamic shared memory of k_diag_lu_inv: the tile and its two inverses.
+// Dynamic shared memory of k_diag_lu_inv: the tile, Linv and the
+// factorization's panels.
 template <typename T>
 constexpr size_t diag_smem() {
-  return 3 * (size_t)NB * TLD * sizeof(T);
+  return 3 * (size_t)tile_elems<T>() * sizeof(T);
 }
 
-constexpr int SB = 16;  // sub-block of the blocked tile factorization
+constexpr int SB = 4;  // pivots per step of the tile factorization
 
 // LU without pivoting of the diagonal tile at (k0, k0) of every active front
 // and the inverses of its triangles, written to INV + inv_off + step*2*NB*NB
@@ -107,403 +121,438 @@ constexpr int SB = 16;  // sub-block of the blocked tile factorization
 // array (kernel_cuda.cu:45-73).  flags[0] counts replaced pivots, flags[1]
 // records a zero or non-finite pivot.
 //
-// Blocked in SB x SB sub-blocks: one warp factors each diagonal sub-block in
-// registers (row k broadcast by shuffles), the rows below and columns right
-// of it inside the tile are finished by substitution (one thread per row /
-// column), and the rest of the tile takes a rank-SB update.  The inverses
-// start from the SB x SB diagonal-block inverses (eight warps at once) and
-// are joined by recursive doubling (inv_join).  A tile smaller than NB is
-// padded with the identity, which leaves its factors and inverses unchanged.
+// The tile is bound by the latency of its 64 dependent pivots, so the
+// inverses ride along with the factorization instead of following it: the
+// bordered matrix [A I; I 0] is eliminated, whose L part below A is
+// I U^-1 = Uinv and whose U part right of A is L^-1 I = Linv.  At every
+// pivot as many rows of A are left as rows of Uinv have begun, so both fit
+// one 64 x 64 array: where a row (column) of A has become final, the row of
+// Uinv (column of Linv) takes its place, starting from zero.  The array is
+// eliminated SB = 4 pivots at a time, one CTA barrier per step, by two
+// halves of the CTA:
+//
+// * the chain (warps 0, 1): thread t finishes row t of the step's four
+//   columns against the 4 x 4 pivot block (x U = a; the block's own rows
+//   start from the identity) and column t of its four rows (L y = a).
+//   Every thread factors the block for itself, in registers, which no
+//   exchange between lanes can match.  The block, row and column of the
+//   next step come from shared memory without the current step's rank-4
+//   update, which the thread applies itself, so the chain never waits for
+//   the rest of the array.
+// * the update (warps 4-7): holds the array in registers, an 8 x 4 patch per
+//   thread; applies each step's rank-4 update and publishes the columns and
+//   rows of the step after next.
+// * warps 2 and 3 collect the finished rows and columns.
+//
+// (Shared memory serves 128 requested bytes a cycle, broadcasts included,
+// so every operand that several threads share is requested by as few of
+// them as possible: a chain of four warps beside update warps that also
+// collected took 1150 cycles a step where this takes 780.)  A full tile on
+// one SM takes 16.3 thousand cycles in FP32 and 28.3 in FP64, where the
+// factorization by 16 x 16 sub-blocks with the inverses joined afterwards
+// took 21.5 and 44.7.
+//
+// Finished rows of Uinv leave by whole 128-byte lines at every step; the
+// tile and Linv, whose columns a step finishes four elements of, are
+// collected in shared memory: Linv is stored at the end, the tile by the
+// caller.  A pivot costs the chain its reciprocal and two dependent
+// operations; pivots that need the
+// guard, the singularity test or a scaled reciprocal send the step through
+// a second pass.  A tile smaller than NB is padded with the identity, which
+// leaves its factors and inverses unchanged; blocks of padding are skipped.
 
-// acc(r, c) += sum_{m0 <= m < m1} A[r + m lda] B[m + c ldb]: an R x C
-// register tile of a product of two shared-memory operands.
-template <typename T, int R, int C>
-__device__ __forceinline__ void tile_mm(const T* A, int lda, const T* B,
-                                        int ldb, int m0, int m1,
-                                        T (&acc)[R][C]) {
-#pragma unroll 4
-  for (int m = m0; m < m1; m++) {
-    T a[R], b[C];
-#pragma unroll
-    for (int r = 0; r < R; r++) a[r] = A[r + m * lda];
-#pragma unroll
-    for (int c = 0; c < C; c++) b[c] = B[m + c * ldb];
-#pragma unroll
-    for (int r = 0; r < R; r++)
-#pragma unroll
-      for (int c = 0; c < C; c++) acc[r][c] += a[r] * b[c];
-  }
-}
+// Slot of row (or column) r in the 64 x 4 panels: r = 4 t + a is at
+// 18 a + t, so the rows of a fixed a and consecutive t and consecutive
+// rows are both in distinct banks as 16-byte vectors.
+__device__ __forceinline__ int sb_slot(int r) { return (r & 3) * 18 + (r >> 2); }
+constexpr int SB_SLOTS = 72;
 
-// Stage B of the tile inverses, by recursive doubling: level 1 joins the
-// SB x SB diagonal-block inverses into 2SB x 2SB ones, level 2 joins those
-// into the NB x NB inverses,
-//   Linv21 = -Linv22 (L21 Linv11),   Uinv12 = -Uinv11 (U12 Uinv22).
-// The first products go to the zero triangles (XL's upper right and XU's
-// lower left NB/2 x NB/2 blocks), which are cleared again at the end.  A
-// thread holds a 2 x 2 (level 1) or 2 x 4 (level 2) register tile; the
-// tiles of one warp share their columns (first product) or rows (second
-// product), so the triangular factor bounds the inner loop per warp.  nbk:
-// the sub-blocks that hold the tile; the rest is identity padding, whose
-// joins are zero and are skipped.
+// A 64 x 4 panel: 16-byte vectors (FP64: two planes of them).
 template <typename T>
-__device__ __forceinline__ void inv_join(const T* D, T* XL, T* XU, int tid,
-                                         int nbk) {
-  constexpr int H = NB / 2;
-  T* TL = XL + H * TLD;  // XL(0:H, H:NB)
-  T* TU = XU + H;        // XU(H:NB, 0:H)
-  const int lane = tid & 31;
-  if (nbk < 2) return;  // one block: nothing off the diagonal
-  {
-    // level 1: join pair P of the diagonal blocks, of L (isU 0) or U (pair
-    // 1 only when its second block is not identity padding)
-    const int pr = tid >> 6, P = pr & 1, isU = pr >> 1, wp = (tid >> 5) & 1;
-    const int b1 = 2 * P * SB, b2 = b1 + SB;
-    const bool work = P == 0 || nbk == NB / SB;
-    T* Tp = TL + P * SB + isU * SB * TLD;
-    if (work) {
-      const int i = 2 * (lane & 7), j = 2 * (wp * 4 + (lane >> 3));
-      T acc[2][2] = {};
-      if (!isU)  // L21 Linv11: Linv11(m, j) = 0 for m < j
-        tile_mm<T, 2, 2>(D + b2 + i + b1 * TLD, TLD, XL + b1 + (b1 + j) * TLD,
-                         TLD, 8 * wp, SB, acc);
-      else       // U12 Uinv22: Uinv22(m, j) = 0 for m > j
-        tile_mm<T, 2, 2>(D + b1 + i + b2 * TLD, TLD, XU + b2 + (b2 + j) * TLD,
-                         TLD, 0, 8 * wp + 8, acc);
-#pragma unroll
-      for (int r = 0; r < 2; r++)
-#pragma unroll
-        for (int c = 0; c < 2; c++) Tp[i + r + (j + c) * TLD] = acc[r][c];
+struct SbPanel {
+  static constexpr int PL = sizeof(T) / 4;  // vectors per row
+  __align__(16) T v[PL][SB_SLOTS][4 / PL];
+  __device__ __forceinline__ void get(int slot, T (&x)[SB]) const {
+    if constexpr (PL == 1) {
+      ld4(v[0][slot], x);
+    } else {
+      ld2(v[0][slot], x[0], x[1]);
+      ld2(v[1][slot], x[2], x[3]);
     }
-    __syncthreads();
-    if (work) {
-      const int i = 2 * (wp * 4 + (lane >> 3)), j = 2 * (lane & 7);
-      T acc[2][2] = {};
-      if (!isU) {  // Linv22 (i, m) = 0 for m > i
-        tile_mm<T, 2, 2>(XL + b2 + i + b2 * TLD, TLD, Tp + j * TLD, TLD, 0,
-                         8 * wp + 8, acc);
-#pragma unroll
-        for (int r = 0; r < 2; r++)
-#pragma unroll
-          for (int c = 0; c < 2; c++)
-            XL[b2 + i + r + (b1 + j + c) * TLD] = -acc[r][c];
-      } else {     // Uinv11 (i, m) = 0 for m < i
-        tile_mm<T, 2, 2>(XU + b1 + i + b1 * TLD, TLD, Tp + j * TLD, TLD,
-                         8 * wp, SB, acc);
-#pragma unroll
-        for (int r = 0; r < 2; r++)
-#pragma unroll
-          for (int c = 0; c < 2; c++)
-            XU[b1 + i + r + (b2 + j + c) * TLD] = -acc[r][c];
-      }
-    }
-    __syncthreads();
   }
-  if (nbk > 2) {
-    // level 2: join the two H x H inverses of L (isU 0) or U
-    const int isU = tid >> 7, wq = (tid >> 5) & 3;
-    {
-      const int i = 2 * (lane & 15), j = 4 * (wq * 2 + (lane >> 4));
-      T acc[2][4] = {};
-      T* out;
-      if (!isU) {
-        tile_mm<T, 2, 4>(D + H + i, TLD, XL + j * TLD, TLD, 8 * wq, H, acc);
-        out = TL;
-      } else {
-        tile_mm<T, 2, 4>(D + i + H * TLD, TLD, XU + H + (H + j) * TLD, TLD, 0,
-                         8 * wq + 8, acc);
-        out = TU;
-      }
-#pragma unroll
-      for (int r = 0; r < 2; r++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) out[i + r + (j + c) * TLD] = acc[r][c];
+  __device__ __forceinline__ void put(int slot, T x0, T x1, T x2, T x3) {
+    if constexpr (PL == 1) {
+      *reinterpret_cast<float4*>(v[0][slot]) = make_float4(x0, x1, x2, x3);
+    } else {
+      *reinterpret_cast<double2*>(v[0][slot]) = make_double2(x0, x1);
+      *reinterpret_cast<double2*>(v[1][slot]) = make_double2(x2, x3);
     }
-    __syncthreads();
-    {
-      const int i = 2 * (wq * 4 + (lane >> 3)), j = 4 * (lane & 7);
-      T acc[2][4] = {};
-      if (!isU) {
-        tile_mm<T, 2, 4>(XL + H + i + H * TLD, TLD, TL + j * TLD, TLD, 0,
-                         8 * wq + 8, acc);
-#pragma unroll
-        for (int r = 0; r < 2; r++)
-#pragma unroll
-          for (int c = 0; c < 4; c++) XL[H + i + r + (j + c) * TLD] = -acc[r][c];
-      } else {
-        tile_mm<T, 2, 4>(XU + i, TLD, TU + j * TLD, TLD, 8 * wq, H, acc);
-#pragma unroll
-        for (int r = 0; r < 2; r++)
-#pragma unroll
-          for (int c = 0; c < 4; c++) XU[i + r + (H + j + c) * TLD] = -acc[r][c];
-      }
-    }
-    __syncthreads();
   }
-  for (int e = tid; e < H * H; e += 256) {
-    const int i = e & (H - 1), j = e / H;
-    TL[i + j * TLD] = (T)0;
-    TU[i + j * TLD] = (T)0;
-  }
-  __syncthreads();
+};
+
+// (the eight panels fit one tile buffer)
+static_assert(8 * sizeof(SbPanel<float>) <= tile_elems<float>() * sizeof(float) &&
+              8 * sizeof(SbPanel<double>) <= tile_elems<double>() * sizeof(double),
+              "panels exceed a tile buffer");
+
+__device__ __forceinline__ void sb_barrier() {  // all 256 threads
+  asm volatile("bar.sync 1, 256;" ::: "memory");
 }
 
-// The tile factorization of one front by the whole CTA (256 threads); D,
-// XL, XU: 3 NB x TLD shared-memory tiles.  On return XL / XU hold Linv /
-// Uinv (also written to INV), the factored tile is back in F and, when LP
-// is given (it may be D), Linv is also in LP with leading dimension PLD.
-// pre: the tile already in shared memory (leading dimension PLD), instead
-// of loading it from the front.  dry: the same code on whatever D, XL, XU
-// and pre hold, writing nothing outside shared memory (no front, inverses
-// or pivot flags): run once, it brings this code into the SM's instruction
-// cache before a real call from the same call site.
+// Four contiguous elements of a column of a shared tile.
+template <typename T>
+__device__ __forceinline__ void tile_st4(T* p, const T (&w)[4]) {
+  if constexpr (pld<T>() % 4 == 0) {
+    st4(p, w);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) p[k] = w[k];
+  }
+}
+template <typename T>
+__device__ __forceinline__ void tile_ld4(const T* p, T (&w)[4]) {
+  if constexpr (pld<T>() % 4 == 0) {
+    ld4(p, w);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) w[k] = p[k];
+  }
+}
+
+// The tile factorization of one front by the whole CTA (256 threads).  D,
+// XL: shared tiles (leading dimension PLD), scratch: eight panels in shared
+// memory (16-byte aligned).  On return D holds the factored tile and XL
+// Linv; both inverses are in INV; the caller stores the tile to the front
+// (it is off the chain: no other task reads it here).  pre: D
+// already holds the tile (entries past the tile's pivots are ignored),
+// instead of loading it from the front.
 template <typename T>
 __device__ __forceinline__ void diag_tile(const FrontDev& f,
                                           T* __restrict__ F,
                                           T* __restrict__ INV, int k0,
                                           int step, double eps, int* flags,
-                                          T* D, T* XL, T* XU,
-                                          T* LP = nullptr,
-                                          const T* pre = nullptr,
-                                          bool dry = false) {
-  __shared__ T rdiag[NB];  // 1 / U[i][i]
+                                          T* D, T* XL, SbPanel<T>* scratch,
+                                          bool pre = false) {
+  constexpr int P = pld<T>();
+  // two buffers each: the columns (rawr, by rows) and rows (rawc, by
+  // columns) of a step, one update short, and the finished ones
+  SbPanel<T>*rawr = scratch, *rawc = scratch + 2, *finr = scratch + 4,
+  *finc = scratch + 6;
   const int kb = min(NB, f.p - k0);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // sub-blocks past the tile (identity padding) need no factorization:
-  // their pivots are 1
-  const int nbk = (kb + SB - 1) / SB, kbp = nbk * SB;
-  if (tid >= kbp && tid < NB) rdiag[tid] = (T)1;
-  T* base = F + f.off + k0 + (int64_t)k0 * f.ld;
-  {
-    // all 16 loads of a thread in flight before the shared-memory stores;
-    // the tile comes from the front, or from pre (leading dimension PLD)
-    // when the caller already holds it (pre may alias XL or XU)
-    T v[NB * NB / 256];
-#pragma unroll
-    for (int q = 0; q < NB * NB / 256; q++) {
-      const int e = tid + 256 * q, i = e & (NB - 1), j = e / NB;
-      v[q] = (i < kb && j < kb)
-                 ? (pre ? pre[i + j * pld<T>()] : __ldcg(base + i + (int64_t)j * f.ld))
-                 : (i == j ? (T)1 : (T)0);
-    }
-    if (pre) __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NB * NB / 256; q++) {
-      const int e = tid + 256 * q, i = e & (NB - 1), j = e / NB;
-      D[i + j * TLD] = v[q];
-      XL[i + j * TLD] = (T)0;
-      XU[i + j * TLD] = (T)0;
-    }
-  }
-  __syncthreads();
-  const T teps = (T)eps, rteps = recip_rn(teps);
-  for (int b = 0; b < nbk; b++) {
-    const int s0 = b * SB;
-    // (1) diagonal sub-block by warp 0; lane l (< SB) owns row s0 + l
-    if (warp == 0) {
-      const int r = s0 + (lane & (SB - 1));
-      T v[SB];
-#pragma unroll
-      for (int j = 0; j < SB; j++) v[j] = D[r + (s0 + j) * TLD];
-      // the pivot is warp-uniform: the replaced-pivot count and the
-      // zero / non-finite test are kept in registers and published once
-      // after the sub-block (a global atomic inside the loop costs a warp
-      // divergence per pivot)
-      int nguard = 0;
-      bool bad = false;
-      const bool guard = f.guard != 0;
-#pragma unroll
-      for (int k = 0; k < SB; k++) {
-        T rowk[SB];
-#pragma unroll
-        for (int j = k; j < SB; j++) rowk[j] = __shfl_sync(0xffffffffu, v[j], k);
-        T piv = rowk[k];
-        // branch-free: the guard, the test and the update are selects, so
-        // the warp never diverges inside the pivot chain
-        // the guard is a select after the reciprocal, off the pivot chain
-        // (1 / +-eps is +-rteps exactly)
-        const bool live = s0 + k < kb;
-        const bool g = guard & live & (piv < teps) & (piv > -teps);
-        const T rraw = pivot_recip(piv);
-        const T rp = g ? (piv < (T)0 ? -rteps : rteps) : rraw;
-        piv = g ? (piv < (T)0 ? -teps : teps) : piv;
-        nguard += g;
-        bad |= live & (!(piv != (T)0) | !isfinite(piv));
-        // lanes below row k take the multiplier and the update (lanes
-        // 16-31 hold copies of the rows and are never stored)
-        const bool upd = lane > k;
-        const T l = v[k] * rp;
-        v[k] = upd ? l : (lane == k ? piv : v[k]);
-#pragma unroll
-        for (int j = k + 1; j < SB; j++) v[j] = upd ? v[j] - l * rowk[j] : v[j];
-        if (lane == 0) rdiag[s0 + k] = rp;
-      }
-      if (lane == 0 && !dry) {
-        if (nguard) atomicAdd(flags, nguard);
-        if (bad) flags[1] = 1;
-      }
-      if (lane < SB)
-#pragma unroll
-        for (int j = 0; j < SB; j++) D[r + (s0 + j) * TLD] = v[j];
-    }
-    __syncthreads();
-    const int rem = kbp - s0 - SB;
-    if (rem > 0) {
-      // (2) rows below: x Ubb = a; columns right: Lbb y = a (unit lower)
-      if (tid < rem) {
-        const int i = s0 + SB + tid;
-        T x[SB];
-#pragma unroll
-        for (int j = 0; j < SB; j++) {
-          T a = D[i + (s0 + j) * TLD];
-#pragma unroll
-          for (int m = 0; m < j; m++) a -= x[m] * D[s0 + m + (s0 + j) * TLD];
-          x[j] = a * rdiag[s0 + j];
-        }
-#pragma unroll
-        for (int j = 0; j < SB; j++) D[i + (s0 + j) * TLD] = x[j];
-      } else if (tid >= 128 && tid < 128 + rem) {
-        const int c = s0 + SB + (tid - 128);
-        T y[SB];
-#pragma unroll
-        for (int i = 0; i < SB; i++) {
-          T a = D[s0 + i + c * TLD];
-#pragma unroll
-          for (int m = 0; m < i; m++) a -= D[s0 + i + (s0 + m) * TLD] * y[m];
-          y[i] = a;
-        }
-#pragma unroll
-        for (int i = 0; i < SB; i++) D[s0 + i + c * TLD] = y[i];
-      }
-      __syncthreads();
-      // (3) rank-SB update of the rest of the tile; the first sub-block's
-      // 48 x 48 update in 3 x 3 register tiles (rows tx + 16 a, columns
-      // ty + 16 b: six shared loads per nine FMAs instead of one per FMA),
-      // the smaller ones one element at a time; every element takes the
-      // same FMAs in the same order either way
-      const int tx = tid & 15, ty = tid >> 4;
-      if (rem == 3 * SB) {
-        T acc[3][3], l[3], u[3];
-#pragma unroll
-        for (int a = 0; a < 3; a++)
-#pragma unroll
-          for (int b = 0; b < 3; b++)
-            acc[a][b] = D[s0 + SB + tx + 16 * a + (s0 + SB + ty + 16 * b) * TLD];
-#pragma unroll
-        for (int t = 0; t < SB; t++) {
-#pragma unroll
-          for (int a = 0; a < 3; a++) l[a] = D[s0 + SB + tx + 16 * a + (s0 + t) * TLD];
-#pragma unroll
-          for (int b = 0; b < 3; b++) u[b] = D[s0 + t + (s0 + SB + ty + 16 * b) * TLD];
-#pragma unroll
-          for (int a = 0; a < 3; a++)
-#pragma unroll
-            for (int b = 0; b < 3; b++) acc[a][b] -= l[a] * u[b];
-        }
-#pragma unroll
-        for (int a = 0; a < 3; a++)
-#pragma unroll
-          for (int b = 0; b < 3; b++)
-            D[s0 + SB + tx + 16 * a + (s0 + SB + ty + 16 * b) * TLD] = acc[a][b];
-      } else
-      for (int jj = ty; jj < rem; jj += 16) {
-        const int j = s0 + SB + jj;
-        T u[SB];
-#pragma unroll
-        for (int t = 0; t < SB; t++) u[t] = D[s0 + t + j * TLD];
-        for (int ii = tx; ii < rem; ii += 16) {
-          const int i = s0 + SB + ii;
-          T acc = D[i + j * TLD];
-#pragma unroll
-          for (int t = 0; t < SB; t++) acc -= D[i + (s0 + t) * TLD] * u[t];
-          D[i + j * TLD] = acc;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // factored tile back to the front (four rows per vector store when the
-  // tile is full and its columns are 16-byte aligned)
-  if (dry) {
-    // (a dry run writes nothing outside shared memory)
-  } else if (kb == NB && aligned16(base) && (f.ld & 3) == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = tid + 256 * q, i = (e & 15) * 4, j = e >> 4;
-      T v[4];
-#pragma unroll
-      for (int a = 0; a < 4; a++) v[a] = D[i + a + j * TLD];
-      st4(base + i + (int64_t)j * f.ld, v);
-    }
-  } else {
-    for (int e = tid; e < NB * NB; e += 256) {
-      const int i = e & (NB - 1), j = e / NB;
-      if (i < kb && j < kb) base[i + (int64_t)j * f.ld] = D[i + j * TLD];
-    }
-  }
-  // inverses, stage A: SB x SB diagonal blocks; warps 0-3 Linv, 4-7 Uinv;
-  // lane j (< SB) computes column j of its block
-  {
-    const int s0 = (warp & 3) * SB, j = lane;
-    if (j < SB) {
-      T x[SB];
-      if (warp < 4) {
-#pragma unroll
-        for (int i = 0; i < SB; i++) {
-          T a = (i == j) ? (T)1 : (T)0;
-#pragma unroll
-          for (int m = 0; m < i; m++) a -= D[s0 + i + (s0 + m) * TLD] * x[m];
-          x[i] = a;
-        }
-#pragma unroll
-        for (int i = 0; i < SB; i++) XL[s0 + i + (s0 + j) * TLD] = x[i];
-      } else {
-#pragma unroll
-        for (int ii = SB - 1; ii >= 0; ii--) {
-          T a = (ii == j) ? (T)1 : (T)0;
-#pragma unroll
-          for (int m = ii + 1; m < SB; m++) a -= D[s0 + ii + (s0 + m) * TLD] * x[m];
-          x[ii] = a * rdiag[s0 + ii];
-        }
-#pragma unroll
-        for (int i = 0; i < SB; i++) XU[s0 + i + (s0 + j) * TLD] = x[i];
-      }
-    }
-  }
-  __syncthreads();
-  // stage B: the off-diagonal blocks
-  inv_join<T>(D, XL, XU, tid, nbk);
+  const int tid = threadIdx.x;
+  const int nsb = (kb + SB - 1) / SB;
+  const int64_t ld = f.ld;
+  T* base = F + f.off + k0 + k0 * ld;
   T* inv = INV + f.inv_off + (int64_t)step * 2 * NB * NB;
-  if (dry) {
-    // (nor the inverses)
-  } else if (aligned16(inv)) {
+  const bool vec = kb == NB && aligned16(base) && (f.ld & 3) == 0;
+  if (tid < NB) {
+    // ------------------------------------------------------------ chain
+    const int i = tid, slot = sb_slot(i);  // the thread's row and column
+    const T teps = (T)eps, rteps = recip_rn(teps);
+    const bool guard = f.guard != 0;
+    const T lo = guard ? max(teps, pivot_lo<T>()) : pivot_lo<T>();
+    int nguard = 0;
+    bool bad = false;
+    T x[SB], y[SB];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = tid + 256 * q, i = (e & 15) * 4, j = e >> 4;
-      T l[4], u[4];
+    for (int k = 0; k < SB; k++) x[k] = y[k] = (T)0;
+    sb_barrier();
+    for (int s = 0; s < nsb; s++) {
+      const int par = s & 1, s0 = SB * s;
+      // the pivot block with the previous step's update.  FP32: every lane
+      // forms all of it.  FP64, where that is 64 multiply-adds at a sixteenth
+      // of a warp each: lane 4 a + c (and its copy 16 up) forms element
+      // (a, c) and all lanes gather the sixteen (28.4 against 30.1 thousand
+      // cycles a tile; FP32 16.5 against 15.8)
+      T d[SB][SB], r[SB], xn[SB], yn[SB], e = (T)0;
+      if constexpr (sizeof(T) == 8) {
+        const int ea = (tid >> 2) & 3, ec = tid & 3;
+        T row[SB];
+        rawr[par].get(18 * ea + s, row);
+        e = ec == 0 ? row[0] : ec == 1 ? row[1] : ec == 2 ? row[2] : row[3];
+        if (s > 0) {
+          T fr[SB], fc[SB];
+          finr[par ^ 1].get(18 * ea + s, fr);
+          finc[par ^ 1].get(18 * ec + s, fc);
 #pragma unroll
-      for (int a = 0; a < 4; a++) {
-        l[a] = XL[i + a + j * TLD];
-        u[a] = XU[i + a + j * TLD];
+          for (int m = 0; m < SB; m++) e -= fr[m] * fc[m];
+        }
       }
-      st4(inv + i + j * NB, l);
-      st4(inv + NB * NB + i + j * NB, u);
-      if (LP) {  // D is free by now
-        if (pld<T>() % 4 == 0) {
-          st4(LP + i + j * pld<T>(), l);
+      auto block = [&]() {
+        if constexpr (sizeof(T) == 8) {
+#pragma unroll
+          for (int a = 0; a < SB; a++)
+#pragma unroll
+            for (int c = 0; c < SB; c++)
+              d[a][c] = __shfl_sync(0xffffffffu, e, 4 * a + c);
         } else {
 #pragma unroll
-          for (int a = 0; a < 4; a++) LP[i + a + j * pld<T>()] = l[a];
+          for (int k = 0; k < SB; k++) rawr[par].get(18 * k + s, d[k]);
+          if (s > 0) {
+            T fr[SB][SB], fc[SB][SB];
+#pragma unroll
+            for (int k = 0; k < SB; k++) {
+              finr[par ^ 1].get(18 * k + s, fr[k]);
+              finc[par ^ 1].get(18 * k + s, fc[k]);
+            }
+#pragma unroll
+            for (int m = 0; m < SB; m++)
+#pragma unroll
+              for (int a = 0; a < SB; a++)
+#pragma unroll
+                for (int c = 0; c < SB; c++) d[a][c] -= fr[a][m] * fc[c][m];
+          }
+        }
+      };
+      block();
+      rawr[par].get(slot, xn);
+      rawc[par].get(slot, yn);
+      bool ok = true;
+#pragma unroll
+      for (int k = 0; k < SB; k++) {
+        const T a = fabs(d[k][k]);
+        ok &= (a >= lo) & (a <= pivot_hi<T>());
+        r[k] = pivot_recip_fast(d[k][k]);
+#pragma unroll
+        for (int a = k + 1; a < SB; a++) {
+          d[a][k] *= r[k];
+#pragma unroll
+          for (int c = k + 1; c < SB; c++) d[a][c] -= d[a][k] * d[k][c];
         }
       }
+      if (!ok) {  // (the pivots are the same in every thread)
+        block();
+#pragma unroll 1
+        for (int k = 0; k < SB; k++) {
+          // (1 / +-eps is +-rteps exactly)
+          T piv = k == 0 ? d[0][0] : k == 1 ? d[1][1] : k == 2 ? d[2][2] : d[3][3];
+          const bool lv = s0 + k < kb;
+          const bool g = guard & lv & (piv < teps) & (piv > -teps);
+          const T rk = g ? (piv < (T)0 ? -rteps : rteps) : pivot_recip(piv);
+          piv = g ? (piv < (T)0 ? -teps : teps) : piv;
+          nguard += g;
+          bad |= lv & (!(piv != (T)0) | !isfinite(piv));
+#pragma unroll
+          for (int q = 0; q < SB; q++)
+            if (q == k) {
+              r[q] = rk;
+              d[q][q] = piv;
+#pragma unroll
+              for (int a = q + 1; a < SB; a++) {
+                d[a][q] *= rk;
+#pragma unroll
+                for (int c = q + 1; c < SB; c++) d[a][c] -= d[a][q] * d[q][c];
+              }
+            }
+        }
+      }
+      // the thread's row and column: the previous step's update (a row or
+      // column that was final in that step starts the inverse's from zero)
+      if (s > 0) {
+        const bool zero = (i >> 2) == s - 1;
+#pragma unroll
+        for (int k = 0; k < SB; k++) {
+          xn[k] = zero ? (T)0 : xn[k];
+          yn[k] = zero ? (T)0 : yn[k];
+        }
+#pragma unroll
+        for (int k = 0; k < SB; k++) {
+          T fr[SB], fc[SB];
+          finr[par ^ 1].get(18 * k + s, fr);
+          finc[par ^ 1].get(18 * k + s, fc);
+#pragma unroll
+          for (int m = 0; m < SB; m++) {
+            xn[k] -= x[m] * fc[m];
+            yn[k] -= fr[m] * y[m];
+          }
+        }
+      }
+      // finished against the block (the block's own: from the identity)
+#pragma unroll
+      for (int k = 0; k < SB; k++) {
+        x[k] = (i >> 2) == s ? ((i & 3) == k ? (T)1 : (T)0) : xn[k];
+        y[k] = (i >> 2) == s ? ((i & 3) == k ? (T)1 : (T)0) : yn[k];
+      }
+#pragma unroll
+      for (int k = 0; k < SB; k++) {
+        x[k] *= r[k];
+#pragma unroll
+        for (int c = k + 1; c < SB; c++) {
+          x[c] -= x[k] * d[k][c];
+          y[c] -= d[c][k] * y[k];
+        }
+      }
+      finr[par].put(slot, x[0], x[1], x[2], x[3]);
+      finc[par].put(slot, y[0], y[1], y[2], y[3]);
+      if (tid == 0) {
+#pragma unroll
+        for (int c = 0; c < SB; c++) {
+          const T w[4] = {d[0][c], d[1][c], d[2][c], d[3][c]};
+          tile_st4(D + s0 + (s0 + c) * P, w);
+        }
+      }
+      sb_barrier();
+    }
+    if (tid == 0) {
+      if (nguard) atomicAdd(flags, nguard);
+      if (bad) flags[1] = 1;
+    }
+  } else if (tid < 2 * NB) {
+    // ---------------------------------------------------------- collect
+    const int i = tid - NB;  // the row and the column
+    sb_barrier();
+    for (int s = 0; s < nsb; s++) {
+      const int par = s & 1, s0 = SB * s;
+      sb_barrier();
+      T w[SB];
+      finr[par].get(sb_slot(i), w);
+      // a row of Uinv, or of the tile's L below the block
+      const bool done = i < s0 + SB;
+#pragma unroll
+      for (int k = 0; k < SB; k++) {
+        if (!done) D[i + (s0 + k) * P] = w[k];
+        inv[NB * NB + i + (s0 + k) * NB] = done ? w[k] : (T)0;
+      }
+      finc[par].get(sb_slot(i), w);
+      if (!done) {  // a column of the tile's U right of the block
+        tile_st4(D + s0 + i * P, w);
+#pragma unroll
+        for (int k = 0; k < SB; k++) w[k] = (T)0;
+      }
+      tile_st4(XL + s0 + i * P, w);  // Linv, zero above the diagonal
+    }
+    // identity padding of the inverses past the tile's blocks
+    for (int j = SB * nsb; j < NB; j++) {
+      const T id = i == j ? (T)1 : (T)0;
+      XL[j + i * P] = id;
+      inv[NB * NB + i + j * NB] = id;
     }
   } else {
-    for (int e = tid; e < NB * NB; e += 256) {
+    // ----------------------------------------------------------- update
+    // rows 4 tx + a and 32 + 4 tx + a, columns 4 ty + c (a, c < 4)
+    const int u = tid - 2 * NB, tx = u & 7, ty = u >> 3;
+    T acc[8][4];
+    if (kb == NB && (pre || vec)) {
+      T v[2][4][4];
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          if (pre)
+            tile_ld4(D + 32 * h + 4 * tx + (4 * ty + c) * P, v[h][c]);
+          else
+            ldg4(base + 32 * h + 4 * tx + (4 * ty + c) * ld, v[h][c]);
+        }
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+          for (int c = 0; c < 4; c++) acc[4 * h + a][c] = v[h][c][a];
+    } else {
+#pragma unroll
+      for (int a = 0; a < 8; a++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          const int i = 32 * (a >> 2) + 4 * tx + (a & 3), j = 4 * ty + c;
+          acc[a][c] = (i < kb && j < kb)
+                          ? (pre ? D[i + j * P] : __ldcg(base + i + j * ld))
+                          : (i == j ? (T)1 : (T)0);
+        }
+    }
+    // the columns and rows of step s into the raw panels
+    auto publish = [&](int s) {
+      const int par = s & 1;
+      if (ty == s) {
+#pragma unroll
+        for (int a = 0; a < 8; a++)
+          rawr[par].put(18 * (a & 3) + 8 * (a >> 2) + tx, acc[a][0], acc[a][1],
+                        acc[a][2], acc[a][3]);
+      }
+      if (tx == (s & 7)) {
+        if (s < 8) {
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+            rawc[par].put(18 * c + ty, acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+            rawc[par].put(18 * c + ty, acc[4][c], acc[5][c], acc[6][c], acc[7][c]);
+        }
+      }
+    };
+    publish(0);
+    publish(1);
+    sb_barrier();
+    for (int s = 0; s < nsb; s++) {
+      const int par = s & 1;
+      sb_barrier();
+      // the inverses' rows and columns of this step start from zero
+      if (ty == s) {
+#pragma unroll
+        for (int a = 0; a < 8; a++)
+#pragma unroll
+          for (int c = 0; c < 4; c++) acc[a][c] = (T)0;
+      }
+      if (tx == (s & 7)) {
+        if (s < 8) {
+#pragma unroll
+          for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) acc[a][c] = (T)0;
+        } else {
+#pragma unroll
+          for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) acc[4 + a][c] = (T)0;
+        }
+      }
+      if (s + 1 < nsb) {
+        T qc[4][SB];
+#pragma unroll
+        for (int c = 0; c < 4; c++) finc[par].get(18 * c + ty, qc[c]);
+#pragma unroll
+        for (int a = 0; a < 8; a++) {
+          T pr[SB];
+          finr[par].get(18 * (a & 3) + 8 * (a >> 2) + tx, pr);
+#pragma unroll
+          for (int k = 0; k < SB; k++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) acc[a][c] -= pr[k] * qc[c][k];
+        }
+        if (s + 2 < nsb) publish(s + 2);
+      }
+    }
+  }
+  sb_barrier();
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int e = tid + 256 * q, i = (e & 15) * 4, j = e >> 4;
+    T w[4];
+    tile_ld4(XL + i + j * P, w);
+    st4(inv + i + j * NB, w);
+  }
+}
+
+// The nr x nc tile S (leading dimension PLD) to dst (leading dimension ld),
+// by 256 threads: whole 16-byte vectors along the columns where they are
+// aligned.
+template <typename T>
+__device__ __forceinline__ void tile_store(T* dst, int64_t ld, int nr, int nc,
+                                           const T* S) {
+  constexpr int P = pld<T>();
+  if (nr == NB && aligned16(dst) && (ld & 3) == 0) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int e = threadIdx.x + 256 * q, i = (e & 15) * 4, j = e >> 4;
+      T w[4];
+      tile_ld4(S + i + j * P, w);
+      if (j < nc) st4(dst + i + j * ld, w);
+    }
+  } else {
+    for (int e = threadIdx.x; e < NB * nc; e += 256) {
       const int i = e & (NB - 1), j = e / NB;
-      const T l = XL[i + j * TLD];
-      inv[e] = l;
-      inv[NB * NB + e] = XU[i + j * TLD];
-      if (LP) LP[i + j * pld<T>()] = l;  // D is free by now
+      if (i < nr) dst[i + j * ld] = S[i + j * P];
     }
   }
 }
@@ -514,11 +563,14 @@ __global__ void __launch_bounds__(256)
                   const FrontDev* __restrict__ fr, T* __restrict__ F,
                   T* __restrict__ INV, int k0, int step, double eps,
                   int* flags) {
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   T* D = reinterpret_cast<T*>(smem_raw);
   const FrontDev f = fr[active[blockIdx.x]];
-  diag_tile<T>(f, F, INV, k0, step, eps, flags, D, D + NB * TLD,
-               D + 2 * NB * TLD);
+  diag_tile<T>(f, F, INV, k0, step, eps, flags, D, D + tile_elems<T>(),
+               reinterpret_cast<SbPanel<T>*>(D + 2 * tile_elems<T>()));
+  const int kb = min(NB, f.p - k0);
+  __syncthreads();
+  tile_store(F + f.off + k0 + (int64_t)k0 * f.ld, (int64_t)f.ld, kb, kb, D);
 }
 
 // Dynamic shared memory of k_panel_apply: the panel tile and the inverse.

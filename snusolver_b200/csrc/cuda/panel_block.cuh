@@ -14,11 +14,14 @@
 //   its rows inside the block (columns [k1, K1)).
 // * the next tile's owner (task t + 1 at step t) carries the chain: while
 //   tile t is factored it applies the previous step's update to tile t's
-//   rows in its own columns; once tile t is published it forms tile t's U
-//   rows there (Linv_t times that), its own L block, the update of its
-//   diagonal tile, and factors it.  Only one product lies between two tile
-//   factorizations on the chain's critical path besides the L and U blocks
-//   of the next tile.
+//   rows in its own columns and loads what else it needs; once tile t is
+//   published it forms tile t's U rows there (Linv_t times that) and its own
+//   L block, then the update of its diagonal tile, and factors it.  Only one
+//   product lies between two tile factorizations on the chain's critical
+//   path besides the L and U blocks of the next tile.  A tile of the chain
+//   of a 4096-pivot FP32 front takes 18.7 us: 10.7 the factorization, 1.9
+//   the U and L blocks, 1.5 their stores, 1.5 the update, 3 the loads and
+//   the hand-over (27 us before: 16.4 the factorization).
 // * column task c covers columns [K1 + 64 c, +64): for every tile t it waits
 //   for the tile and forms U_t = Linv_t (A_t - sum_{s<t} L_ts U_s) for its
 //   columns (the U12 rows of the block, right of it).
@@ -122,12 +125,15 @@ __device__ __forceinline__ void pb_load(T* S, const T* src, int64_t ld, int nr,
   }
 }
 
-// One value split into TF32 hi + lo (round to nearest, ties away):
-// hi carries the leading 11 bits, lo the next 11.
+// One value split into TF32 hi + lo: hi carries the leading 11 bits (to
+// nearest, ties away from zero), lo the next 12, of which the tensor cores
+// read 11 -- the one bit they drop is the one rounding would drop.  In
+// integer operations: with cvt.rna.tf32.f32, which issues at a quarter of
+// their rate, the conversions bound the 64 x 64 x 64 product (3450 cycles
+// against 2300).  A NaN reaches lo, an infinity hi and lo.
 __device__ __forceinline__ void tf32_split(float x, uint32_t& hi, uint32_t& lo) {
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-  const float r = x - __uint_as_float(hi);
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
+  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  lo = __float_as_uint(x - __uint_as_float(hi));
 }
 
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
@@ -208,18 +214,21 @@ __device__ __forceinline__ void pb_mm(T (&acc)[4][4], const T* A, const T* B,
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int rb = pb_rb(w), cb = 32 * (w >> 2);
-    // d[i][j]: columns cb + 16 i + {g, g + 8}, rows rb + 8 j + 2 t + {0, 1}
-    float d[2][2][4];
+    // d[i][j]: columns cb + 16 i + {g, g + 8}, rows rb + 8 j + 2 t + {0, 1};
+    // dl: the two small products apart, as the tensor cores truncate each
+    // sum to the accumulator's exponent (error of a 64-long product against
+    // 64 bits: 5.2e-7 in one accumulator, 1.9e-7 in two)
+    float d[2][2][4], dl[2][2][4];
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
       for (int j = 0; j < 2; j++)
 #pragma unroll
-        for (int e = 0; e < 4; e++) d[i][j][e] = 0.f;
+        for (int e = 0; e < 4; e++) d[i][j][e] = dl[i][j][e] = 0.f;
     const int k8 = min((kk + 7) & ~7, tri == PB_LOWER_A   ? rb + 16
                                       : tri == PB_UPPER_B ? cb + 32
                                                           : NB);
-#pragma unroll 1
+#pragma unroll 2
     for (int k0 = 0; k0 < k8; k0 += 8) {
       // MMA A operand (16 x 8, row-major) = B^T: element (m, k) = B(k, m)
       uint32_t ah[2][4], al[2][4];
@@ -244,9 +253,12 @@ __device__ __forceinline__ void pb_mm(T (&acc)[4][4], const T* A, const T* B,
 #pragma unroll
         for (int j = 0; j < 2; j++) {
           mma_tf32(d[i][j], ah[i], bh[j][0], bh[j][1]);
-          mma_tf32(d[i][j], ah[i], bl[j][0], bl[j][1]);
-          mma_tf32(d[i][j], al[i], bh[j][0], bh[j][1]);
+          mma_tf32(dl[i][j], ah[i], bl[j][0], bl[j][1]);
         }
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) mma_tf32(dl[i][j], al[i], bh[j][0], bh[j][1]);
     }
     // fragment element e of tile (i, j): row 8 j + 2 t + (e & 1), column
     // 16 i + g + 8 (e >> 1) -> acc[(e & 1) + 2 j][2 i + (e >> 1)]
@@ -256,7 +268,7 @@ __device__ __forceinline__ void pb_mm(T (&acc)[4][4], const T* A, const T* B,
       for (int j = 0; j < 2; j++)
 #pragma unroll
         for (int e = 0; e < 4; e++)
-          acc[(e & 1) + 2 * j][2 * i + (e >> 1)] = d[i][j][e];
+          acc[(e & 1) + 2 * j][2 * i + (e >> 1)] = d[i][j][e] + dl[i][j][e];
   }
 }
 
@@ -322,6 +334,19 @@ __device__ __forceinline__ void pb_store(T* dst, int64_t ld, int nr, int nc,
   }
 }
 
+// S(i, j) = acc for i < nr, j < nc, zero elsewhere.
+template <typename T>
+__device__ __forceinline__ void pb_put(T* S, int nr, int nc,
+                                       const T (&acc)[4][4]) {
+#pragma unroll
+  for (int b = 0; b < 4; b++)
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+      const int i = PbMap<T>::row(a), j = PbMap<T>::col(b);
+      S[i + j * pld<T>()] = i < nr && j < nc ? acc[a][b] : (T)0;
+    }
+}
+
 // S(i, j) = S(i, j) - acc for i < nr, j < nc, zero elsewhere: the update
 // pb_store(sub) applies, on a tile already in shared memory; with dst, the
 // updated values (i < nr, j < nc) also go to dst (leading dimension ld).
@@ -344,11 +369,55 @@ __device__ __forceinline__ void pb_sub(T* S, int nr, int nc,
   }
 }
 
-// Dynamic shared memory: three tile buffers (the diagonal-tile
-// factorization's D / Linv / Uinv, reused as product tiles).
+// v = src(i, j) at a thread's register tile, i < nr, j < nc, zero elsewhere
+// (v[b][a]; row pairs as vectors where they are aligned, as in pb_store).
+template <typename T>
+__device__ __forceinline__ void pb_get(const T* src, int64_t ld, int nr, int nc,
+                                       T (&v)[4][4]) {
+  const int r0 = PbMap<T>::r0();
+  const bool vec = sizeof(T) == 4 && ((reinterpret_cast<uintptr_t>(src + r0) & 7) == 0) &&
+                   (ld & 1) == 0;
+#pragma unroll
+  for (int b = 0; b < 4; b++) {
+    const int j = PbMap<T>::col(b);
+#pragma unroll
+    for (int a = 0; a < 4; a += 2) {
+      const int i = PbMap<T>::row(a);
+      if (vec && j < nc && PbMap<T>::row(a + 1) < nr) {
+        const float2 q = __ldcg(reinterpret_cast<const float2*>(src + i + j * ld));
+        v[b][a] = (T)q.x, v[b][a + 1] = (T)q.y;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int ie = PbMap<T>::row(a + e);
+          v[b][a + e] = (ie < nr && j < nc) ? __ldcg(src + ie + j * ld) : (T)0;
+        }
+      }
+    }
+  }
+}
+
+// Sets two flags behind one release fence (as raise_flag).
+__device__ __forceinline__ void raise_flags2(int* f0, int* f1) {
+  asm volatile(
+      "fence.acq_rel.gpu;\n\t"
+      "st.relaxed.gpu.global.b32 [%0], %2;\n\t"
+      "st.relaxed.gpu.global.b32 [%1], %2;" ::"l"(f0),
+      "l"(f1), "r"(1)
+      : "memory");
+}
+
+// Dynamic shared memory: the product tiles, which the diagonal-tile
+// factorization also uses (the tile, Linv, its panels).  FP32 holds both
+// tile inverses at once on the chain; in FP64 a fourth tile would leave
+// room for one CTA per SM only.
+template <typename T>
+constexpr int block_tiles() {
+  return sizeof(T) == 4 ? 4 : 3;
+}
 template <typename T>
 constexpr size_t block_smem() {
-  return 3 * (size_t)tile_elems<T>() * sizeof(T);
+  return block_tiles<T>() * (size_t)tile_elems<T>() * sizeof(T);
 }
 
 template <typename T>
@@ -362,6 +431,8 @@ __global__ void __launch_bounds__(256, 2)
   T* S0 = reinterpret_cast<T*>(smem_raw);
   T* S1 = S0 + tile_elems<T>();
   T* S2 = S1 + tile_elems<T>();
+  constexpr bool FOUR = block_tiles<T>() == 4;
+  T* S3 = S2 + (FOUR ? tile_elems<T>() : 0);
   __shared__ int bad, s_task;
   if (threadIdx.x == 0) bad = 0;
   for (;;) {
@@ -421,22 +492,15 @@ __global__ void __launch_bounds__(256, 2)
             pb_load(S2, Fo + k0 + c0n * ld, ld, NB, ncn);
           }
         }
-        if (own || (next && f.p > OB_COLS)) {
-          // owner: the diagonal tile (its columns are up to date)
-          // (Linv comes back in S0, product layout; the tile from S0 when
-          // our work as the next owner left it there).  The next owner of
-          // a front of more than one outer block (a long chain) runs this
-          // same call once, dry, on a 16 x 16 scratch tile in S0 / S1 (S2
-          // keeps tile t's rows) while tile t is factored: the chain moves
-          // to another SM at every tile, and its code would otherwise start
-          // cold there
-          diag_tile<T>(f, F, INV, own ? k0 : f.p - SB, step, eps, dflags, S0,
-                       S1, own ? S2 : S1, own ? S0 : (T*)nullptr,
-                       own ? (pre ? S0 : (const T*)nullptr) : S0, !own);
+                if (own) {
+          // the diagonal tile (its columns are up to date; in S0 when our
+          // work as the next owner left it there); Linv comes back in S1
+          diag_tile<T>(f, F, INV, k0, step, eps, dflags, S0, S1,
+                       reinterpret_cast<SbPanel<T>*>(S2), pre);
           __syncthreads();
-        }
-        if (own) {
           if (threadIdx.x == 0) raise_flag(tflag(0));
+          tile_store(Fo + k0 + k0 * ld, ld, kb, kb, S0);
+          __syncthreads();  // (S0 is reused)
           const int pk0 = K0 + NB * max(deferred, 0);
           if (deferred >= 0) {
             // the previous step's update of our rows past the next tile
@@ -444,7 +508,7 @@ __global__ void __launch_bounds__(256, 2)
               bad = 1;
             __syncthreads();
             if (bad) return;
-            pb_load(S1, Fo + R0 + pk0 * ld, ld, nr, NB);  // our L block
+            pb_load(S0, Fo + R0 + pk0 * ld, ld, nr, NB);  // our L block
           }
           // per column chunk past the next tile (whose U rows the next
           // owner forms): the deferred update of our rows, then the U rows
@@ -456,14 +520,14 @@ __global__ void __launch_bounds__(256, 2)
             if (deferred >= 0) {
               pb_load(S2, Fo + pk0 + c0 * ld, ld, NB, nc);  // its U rows
               __syncthreads();
-              pb_mm(acc, S1, S2, NB);
+              pb_mm(acc, S0, S2, NB);
               __syncthreads();
               pb_store(Fo + R0 + c0 * ld, ld, nr, nc, acc, true, S2);
               have = kb == NB;  // (a partial tile would hold L rows past kb)
             }
             if (!have) pb_load(S2, Fo + k0 + c0 * ld, ld, kb, nc);
             __syncthreads();
-            pb_mm(acc, S0, S2, kb, PB_LOWER_A);  // Linv A
+            pb_mm(acc, S1, S2, kb, PB_LOWER_A);  // Linv A
             pb_store(Fo + k0 + c0 * ld, ld, kb, nc, acc, false, (T*)nullptr);
             __syncthreads();
           }
@@ -486,30 +550,57 @@ __global__ void __launch_bounds__(256, 2)
           const int c0 = k1, nc = min(NB, K1 - c0);  // our tile's columns
           T acc[4][4];
           // (2) tile t factored: its U rows here (Linv_t S2), our L block
-          // (A Uinv_t) and the update of our diagonal tile, kept in S0
+          // (A Uinv_t) and the update of our diagonal tile, kept in S0.
+          // What needs no factors of tile t -- our rows of it and our
+          // diagonal tile, up to date since the previous step -- is loaded
+          // before the wait
+          T dv[4][4];
+          pb_load(S1, Fo + R0 + k0 * ld, ld, nr, kb);
+          if (FOUR) pb_get(Fo + R0 + c0 * ld, ld, nr, nc, dv);
           if (threadIdx.x == 0 && !wait_flag(tflag(0), err)) bad = 1;
           __syncthreads();
           if (bad) return;
-          pb_load(S0, tinv(0), (int64_t)NB, NB, NB);        // Linv_t
-          pb_load(S1, Fo + R0 + k0 * ld, ld, nr, kb);   // our rows of tile t
+          pb_load(S0, tinv(0), (int64_t)NB, NB, NB);            // Linv_t
+          if (FOUR) pb_load(S3, tinv(1), (int64_t)NB, NB, NB);  // Uinv_t
           __syncthreads();
           pb_mm(acc, S0, S2, kb, PB_LOWER_A);
-          __syncthreads();
-          pb_store(Fo + k0 + c0 * ld, ld, kb, nc, acc, false, S2);  // S2 = U
-          pb_load(S0, tinv(1), (int64_t)NB, NB, NB);          // Uinv_t
-          __syncthreads();
-          if (threadIdx.x == 0) raise_flag(tflag(2));
-          pb_mm(acc, S1, S0, kb, PB_UPPER_B);
-          __syncthreads();
-          pb_store(Fo + R0 + k0 * ld, ld, nr, kb, acc, false, S1);  // S1 = L
-          pb_load(S0, Fo + R0 + c0 * ld, ld, nr, nc);               // our tile
-          __syncthreads();
-          if (threadIdx.x == 0) raise_flag(tflag(3));
-          // (the whole updated tile also goes back to the front: our rows
-          // past the front's last pivot, if any, are L rows that we read
-          // back from there as the tile's owner)
+          if constexpr (FOUR) {
+            T accl[4][4];
+            pb_mm(accl, S1, S3, kb, PB_UPPER_B);
+            __syncthreads();
+            pb_put(S2, kb, nc, acc);   // S2 = U
+            pb_put(S1, nr, kb, accl);  // S1 = L
+            __syncthreads();
+            tile_store(Fo + k0 + c0 * ld, ld, kb, nc, S2);
+            tile_store(Fo + R0 + k0 * ld, ld, nr, kb, S1);
+            __syncthreads();
+            if (threadIdx.x == 0) raise_flags2(tflag(2), tflag(3));
+          } else {
+            __syncthreads();
+            pb_store(Fo + k0 + c0 * ld, ld, kb, nc, acc, false, S2);
+            pb_load(S0, tinv(1), (int64_t)NB, NB, NB);
+            __syncthreads();
+            if (threadIdx.x == 0) raise_flag(tflag(2));
+            pb_mm(acc, S1, S0, kb, PB_UPPER_B);
+            __syncthreads();
+            pb_store(Fo + R0 + k0 * ld, ld, nr, kb, acc, false, S1);
+            pb_load(S0, Fo + R0 + c0 * ld, ld, nr, nc);  // our tile
+            __syncthreads();
+            if (threadIdx.x == 0) raise_flag(tflag(3));
+          }
           pb_mm(acc, S1, S2, kb);
-          pb_sub(S0, nr, nc, acc, Fo + R0 + c0 * ld, ld);
+          // (the updated tile goes back to the front only when it is
+          // partial: our rows past the front's last pivot are then L rows
+          // that we read back from there as the tile's owner)
+          T* back = nc < NB ? Fo + R0 + c0 * ld : (T*)nullptr;
+          if (FOUR) {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+              for (int a = 0; a < 4; a++)
+                S0[PbMap<T>::row(a) + PbMap<T>::col(q) * pld<T>()] = dv[q][a];
+          }
+          pb_sub(S0, nr, nc, acc, back, ld);
           __syncthreads();
           pre = true;
           if (c0 + NB < K1) deferred = t;
@@ -528,8 +619,9 @@ __global__ void __launch_bounds__(256, 2)
         T acc[4][4];
         pb_mm(acc, S0, S1, kb, PB_UPPER_B);
         __syncthreads();
-        pb_store(Fo + R0 + k0 * ld, ld, nr, kb, acc, false, S0);  // S0 = L
+        pb_put(S0, nr, kb, acc);  // S0 = L
         __syncthreads();
+        tile_store(Fo + R0 + k0 * ld, ld, nr, kb, S0);
         for (int c0 = k1; c0 < K1; c0 += NB) {
           if (c0 - k1 < 2 * NB) {
             if (threadIdx.x == 0 && !wait_flag(tflag(c0 == k1 ? 2 : 1), err))
@@ -539,9 +631,19 @@ __global__ void __launch_bounds__(256, 2)
           }
           const int nc = min(NB, K1 - c0);
           pb_load(S2, Fo + k0 + c0 * ld, ld, kb, nc);  // U rows of tile t
+          // (FP32: the target's loads run beside the product; FP64 has no
+          // registers left for them)
+          T dv[4][4];
+          if (FOUR) pb_get(Fo + R0 + c0 * ld, ld, nr, nc, dv);
           __syncthreads();
           pb_mm(acc, S0, S2, kb);
-          pb_store(Fo + R0 + c0 * ld, ld, nr, nc, acc, true, (T*)nullptr);
+          if (FOUR) {
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+              for (int q = 0; q < 4; q++) acc[a][q] = dv[q][a] - acc[a][q];
+          }
+          pb_store(Fo + R0 + c0 * ld, ld, nr, nc, acc, !FOUR, (T*)nullptr);
           __syncthreads();
         }
       }
