@@ -388,7 +388,7 @@ class CudaEngine : public Engine {
     invtot_ = ioff;
     int rc;
     {
-      // one flag per pivot tile of every front, for each sweep direction
+      // first flag of every front (flags per pivot tile)
       std::vector<int64_t> fo(std::max(nfronts_, 1), 0);
       int64_t acc = 0;
       for (int f = 0; f < nfronts_; f++) {
@@ -397,12 +397,9 @@ class CudaEngine : public Engine {
       }
       ntileflags_ = std::max<int64_t>(acc, 1);
       if ((rc = upload(d_flag_off_, fo))) return rc;
-      // solve sweeps: one flag per tile and direction, then one task
-      // counter per level and direction
+      // solve sweeps: one task counter per level and direction
       // (two sets of counters: a distributed run sweeps two schedules)
-      // (per column group of a pass: SWEEP_GROUPS sets of tile flags)
-      tflags_size_ =
-          2 * SWEEP_GROUPS * ntileflags_ + 4 * (int64_t)nlevels_ + 2;
+      tflags_size_ = 4 * (int64_t)nlevels_ + 2;
       if ((rc = alloc(d_tflags_, (size_t)tflags_size_))) return rc;
       // fused panel path: four flags per tile, then one task counter per
       // outer-block launch (a level has no more outer blocks than tiles)
@@ -745,6 +742,7 @@ class CudaEngine : public Engine {
       // every work vector zero; the shared fronts' pivot rows start from B
       // on rank 0 only, so the sum over the ranks holds B once
       CK(cudaMemsetAsync(W, 0, sizeof(T) * wtot_ * nrhs, st));
+      CK(cudaMemsetAsync(Y, 0xff, sizeof(T) * ytot_ * nrhs, st));  // (SweepNan)
       if (opt_.dist_rank == 0 && nslist_) {
         k_solve_init<T><<<SOLVE_SPLIT * nslist_, 256, 0, st>>>(
             d_slist_, d_fr_, d_gidx_, dB, ldb, nrhs, W);
@@ -1039,15 +1037,11 @@ class CudaEngine : public Engine {
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int* fl = d_tflags_ + (fwd ? 0 : SWEEP_GROUPS * ntileflags_);
-    int* ctr = d_tflags_ + 2 * SWEEP_GROUPS * ntileflags_ + ctr_off_ +
-               2 * std::max(cur_level_, 0) + (fwd ? 0 : 1);
+    int* ctr = d_tflags_ + ctr_off_ + 2 * std::max(cur_level_, 0) + (fwd ? 0 : 1);
     ++launches_;
     CK(cudaLaunchKernelEx(&cfg, k, tasks, ntasks, ngroups,
-                          (const FrontDev*)d_fr_, F, I,
-                          (const int64_t*)d_flag_off_, (int64_t)ntileflags_,
-                          nrhs, W, Y, (const int*)d_gidx_, X, ldx, fl, ctr,
-                          d_flags_ + 4));
+                          (const FrontDev*)d_fr_, F, I, nrhs, (const T*)W, Y,
+                          (const int*)d_gidx_, X, ldx, ctr, d_flags_ + 4));
     return ENG_OK;
   }
   template <typename T, int R>
@@ -1085,15 +1079,13 @@ class CudaEngine : public Engine {
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int* flags = d_sctl_ + (fwd ? 0 : ntileflags_);
-    int* ctr = d_sctl_ + 2 * ntileflags_;
+    int* ctr = d_sctl_;
     int* next = ctr + 3 * (int64_t)nfronts_ + (fwd ? 0 : 1);
     ++launches_;
     CK(cudaLaunchKernelEx(&cfg, k, (const SolveTask*)(fwd ? d_fwd_tasks_ : d_bwd_tasks_),
                           ntasks, (const FrontDev*)d_fr_, (const SweepDep*)d_dep_,
-                          (const int*)d_gidx_, F, I, (const int64_t*)d_flag_off_,
-                          nfronts_, nrhs, n_, Z, Y, X, ldx, flags, ctr, next,
-                          d_flags_ + 4));
+                          (const int*)d_gidx_, F, I, nfronts_, nrhs, n_, Z, Y, X,
+                          ldx, ctr, next, d_flags_ + 4));
     return ENG_OK;
   }
   template <typename T>
@@ -2193,6 +2185,7 @@ class CudaEngine : public Engine {
     cur_level_ = -1;
     int pi = prof_begin(KF_SWEEP, st);
     CK(cudaMemsetAsync(d_sctl_, 0, sizeof(int) * sctl_size_, st));
+    CK(cudaMemsetAsync(Y, 0xff, sizeof(T) * ytot_ * nrhs, st));  // (SweepNan)
     const int64_t tot = (int64_t)n_ * nrhs;
     k_sweep_init<T><<<(int)((tot + 255) / 256), 256, 0, st>>>(n_, nrhs, B, ldb, W);
     CKL();
@@ -2201,6 +2194,7 @@ class CudaEngine : public Engine {
     prof_end(pi, KF_SWEEP, st, 2.0 * sweep_elems_ * nrhs,
              sweep_elems_ * es + (es + 8.0) * tot);
     pi = prof_begin(KF_SWEEP, st);
+    CK(cudaMemsetAsync(W, 0xff, sizeof(T) * ytot_ * nrhs, st));  // (SweepNan)
     if ((rc = fused_launch<T>(false, F, I, nrhs, W, Y, X, ldx, st))) return rc;
     prof_end(pi, KF_SWEEP, st, 2.0 * sweep_elems_ * nrhs,
              sweep_elems_ * es + 8.0 * tot);
@@ -2266,7 +2260,7 @@ class CudaEngine : public Engine {
     if ((rc = upload(d_dep_, dep))) return rc;
     if ((rc = upload(d_fwd_tasks_, fw))) return rc;
     if ((rc = upload(d_bwd_tasks_, bw))) return rc;
-    sctl_size_ = 2 * ntileflags_ + 3 * (int64_t)nf + 2;
+    sctl_size_ = 3 * (int64_t)nf + 2;
     return alloc(d_sctl_, (size_t)sctl_size_);
   }
 
@@ -2278,6 +2272,7 @@ class CudaEngine : public Engine {
       return ENG_EINVAL;
     }
     CK(cudaMemsetAsync(d_tflags_, 0, sizeof(int) * tflags_size_, st));
+    CK(cudaMemsetAsync(Y, 0xff, sizeof(T) * ytot_ * nrhs, st));  // (SweepNan)
     int rc;
     if ((rc = sweep_levels<T>(lv_, 0, true, true, F, I, W, Y, B, ldb, X, ldx,
                               nrhs, st)))
@@ -2341,7 +2336,7 @@ class CudaEngine : public Engine {
         if (L.ngl) {
           pi = prof_begin(KF_SOLVE_GEMM, st);
           SNU_RG_DISPATCH(nrhs, k_gemv_l21, T, (L.ngl * col_groups(nrhs), 256, 0, st),
-                          (L.gl, L.ngl, d_fr_, F, nrhs, W, Y));
+                          (L.gl, col_groups(nrhs), d_fr_, F, nrhs, W, Y));
           CKL();
           prof_end(pi, KF_SOLVE_GEMM, st, 2.0 * L.gq_elems * nrhs,
                    L.gq_elems * es);
@@ -2361,7 +2356,7 @@ class CudaEngine : public Engine {
         if (L.ngq) {
           pi = prof_begin(KF_SOLVE_GEMM, st);
           SNU_RG_DISPATCH(nrhs, k_gemv_u12, T, (L.ngq * col_groups(nrhs), 256, 0, st),
-                          (L.gq, L.ngq, d_fr_, F, nrhs, W, Y));
+                          (L.gq, col_groups(nrhs), d_fr_, F, nrhs, W, Y));
           CKL();
           prof_end(pi, KF_SOLVE_GEMM, st, 2.0 * L.gq_elems * nrhs,
                    L.gq_elems * es);
@@ -2861,7 +2856,8 @@ class CudaEngine : public Engine {
   size_t wcap64_ = 0, wcap32_ = 0, ycap64_ = 0, ycap32_ = 0, rcapR_ = 0,
          rcapD_ = 0;
   int64_t ytot_ = 0, invtot_ = 0;
-  // pivot-block sweep flags (forward, then backward) and per-front offsets
+  // first tile flag of every front (panel kernel); task counters of the
+  // pivot-block sweeps
   int64_t* d_flag_off_ = nullptr;
   int* d_tflags_ = nullptr;
   int64_t tflags_size_ = 0;
@@ -2908,7 +2904,7 @@ class CudaEngine : public Engine {
   SolveTask* d_bwd_tasks_ = nullptr;
   int nfwd_ = 0, nbwd_ = 0;
   SweepDep* d_dep_ = nullptr;
-  int* d_sctl_ = nullptr;  // tile flags (both directions), counters, task counters
+  int* d_sctl_ = nullptr;  // counters per front, task counters
   int64_t sctl_size_ = 0;
   double sweep_elems_ = 0;  // factor entries one sweep reads (per column)
   int force_tcp_ = -1;  // tensor-core kernel variant forced (-1: per batch)

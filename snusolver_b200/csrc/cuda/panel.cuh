@@ -78,7 +78,7 @@ __device__ __forceinline__ double recip_rn(double x) { return __drcp_rn(x); }
 // Newton-Raphson step in its FMA form, e = 1 - x r0, r = r0 + r0 e
 // (Markstein, "IA-64 and Elementary Functions", 2000): the refined value
 // is within one ulp of the correctly rounded reciprocal and nearly always
-// equal to it (snu_check_pivot_reciprocal measures both on the GPU).  The
+// equal to it (snu_selftest_pivot_reciprocal measures both on the GPU).  The
 // .ftz form is one instruction, where the form that keeps subnormals added
 // 55 cycles to every pivot; pivots whose value or reciprocal it could flush
 // (outside [2^-120, 2^120]) take the same steps on a scaled pivot, in

@@ -7,11 +7,12 @@
 //
 // * the pivot block (rows and columns [0, p)): one cooperative launch over
 //   (front, 128-row chunk) tasks.  The chunk holding a tile's rows solves the
-//   tile with the stored inverse of the diagonal tile, writes the result to Y
-//   and raises the tile's flag; the other chunks of the front wait for the
-//   flag (bounded spin), read the tile's solution and update their rows.
-//   The factor columns a chunk needs for a tile are staged into shared
-//   memory with cp.async while it waits.
+//   tile with the stored inverse of the diagonal tile and publishes the
+//   result in Y; the other chunks of the front wait for it (bounded spin) and
+//   update their rows.  Y itself is the flag: it starts as a NaN that no
+//   result is stored as (SweepNan), and a waiting thread spins on the
+//   elements that it needs.  The factor columns a chunk needs for a tile are
+//   staged into shared memory with cp.async while it waits.
 // * the off-diagonal part (L21 y for the forward sweep, U12 x_Q for the
 //   backward sweep): a tall-skinny product over (front, 64-row, 256-column)
 //   blocks that adds into W with atomics.
@@ -23,9 +24,8 @@ namespace snu {
 constexpr int RG = 16;          // right-hand sides per register group
 // columns per pass of the level-by-level sweeps: the pivot-block sweeps run
 // the pass's register groups as independent task chains of one launch (a
-// group's tasks after the previous group's), each with its own tile flags
+// group's tasks after the previous group's)
 constexpr int SOLVE_COLS = 64;
-constexpr int SWEEP_GROUPS = SOLVE_COLS / RG;
 constexpr int DIAG_ROWS = 128;  // rows of a pivot-block chunk (= threads)
 constexpr long WAVE_SPIN_LIMIT = 1L << 22;
 
@@ -103,294 +103,397 @@ __device__ __forceinline__ void stage_inv(T* Xs, const T* inv) {
     cp_async16(Xs + e * V, inv + e * V);
 }
 
-// out[i][r] = sum_m Xs[i + m NB] in[m][r] for the kb x nr block; written to
-// Yf (ld p) as well.  Called by all DIAG_ROWS threads of the CTA.  Thread
-// t takes row i = t % NB and columns r = t / NB + (DIAG_ROWS / NB) q: its
-// dot products share row i of the inverse and run side by side, each
-// summed over m in order.
-template <typename T, int R>
-__device__ __forceinline__ void tile_apply(const T* Xs, T (*in)[R],
-                                           T (*out)[R], T* Yf, int ldy, int k0,
-                                           int kb, int r0, int nr) {
-  static_assert(DIAG_ROWS % NB == 0, "a chunk is whole tiles");
-  constexpr int RS = DIAG_ROWS / NB, PER = (R + RS - 1) / RS;
-  const int i = threadIdx.x % NB, rb = threadIdx.x / NB;
-  T a[PER];
-#pragma unroll
-  for (int q = 0; q < PER; q++) a[q] = (T)0;
-#pragma unroll 8
-  for (int m = 0; m < NB; m++) {
-    const T x = Xs[i + m * NB];
-#pragma unroll
-    for (int q = 0; q < PER; q++)
-      if (rb + RS * q < R) a[q] += x * in[m][rb + RS * q];
+// The NaN that marks an element of Y that is not solved yet: every bit set,
+// so a buffer is marked by a memset.  A result with those bits (a NaN that
+// came in with the right-hand side) is published as the usual NaN instead.
+template <typename T>
+struct SweepNan;
+template <>
+struct SweepNan<float> {
+  __device__ __forceinline__ static float mark() { return __uint_as_float(0xffffffffu); }
+  __device__ __forceinline__ static bool is(float v) { return __float_as_uint(v) == 0xffffffffu; }
+  __device__ __forceinline__ static float load(const float* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return __uint_as_float(v);
   }
+  __device__ __forceinline__ static void publish(float* p, float v) {
+    const uint32_t b = is(v) ? 0x7fffffffu : __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(b) : "memory");
+  }
+};
+template <>
+struct SweepNan<double> {
+  __device__ __forceinline__ static double mark() { return __longlong_as_double(-1ll); }
+  __device__ __forceinline__ static bool is(double v) { return __double_as_longlong(v) == -1ll; }
+  __device__ __forceinline__ static double load(const double* p) {
+    long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return __longlong_as_double(v);
+  }
+  __device__ __forceinline__ static void publish(double* p, double v) {
+    const long long b = is(v) ? 0x7fffffffffffffffll : __double_as_longlong(v);
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
+  }
+};
+
+// v[q] = src[off(q)] for the q that are wanted, once published (bounded
+// spin; all loads in flight together); on timeout sets *err and returns
+// false.
+template <typename T, int N, typename Off>
+__device__ __forceinline__ bool poll_all(const T* src, Off off, T (&v)[N],
+                                         int* err) {
+  bool again = true;
+  for (long it = 0; again && it < WAVE_SPIN_LIMIT; it++) {
+    again = false;
 #pragma unroll
-  for (int q = 0; q < PER; q++) {
-    const int r = rb + RS * q;
-    if (r < R) {
-      const bool ok = i < kb && r < nr;
-      out[i][r] = ok ? a[q] : (T)0;
-      if (ok) Yf[k0 + i + (int64_t)(r0 + r) * ldy] = a[q];
+    for (int q = 0; q < N; q++) {
+      const int64_t o = off(q);
+      if (o >= 0 && (it == 0 || SweepNan<T>::is(v[q]))) v[q] = SweepNan<T>::load(src + o);
     }
+#pragma unroll
+    for (int q = 0; q < N; q++) again |= off(q) >= 0 && SweepNan<T>::is(v[q]);
+    if (again && it > 4) __nanosleep(20);
+  }
+  if (again) atomicExch(err, 1);
+  return !again;
+}
+
+// Shared memory of a pivot-block chunk beside the staging buffers: a tile's
+// solution and right-hand side, [NB][R] with padded rows.
+template <typename T, int R>
+struct ChunkSmem {
+  static constexpr int RS = R >= 8 ? R + 16 / (int)sizeof(T) : R;
+  __align__(16) T ys[NB][RS];
+  __align__(16) T ws[NB][RS];
+  int bad;
+};
+
+// N contiguous values from shared memory, as wide as N allows (aligned to
+// N values, N a power of two).
+template <int N, typename T>
+__device__ __forceinline__ void lds(const T* p, T (&v)[N]) {
+  constexpr int V = 16 / sizeof(T);
+  if constexpr (N >= V) {
+#pragma unroll
+    for (int q = 0; q < N; q += V) {
+      const uint4 t = *reinterpret_cast<const uint4*>(p + q);
+      if constexpr (sizeof(T) == 4) {
+        v[q] = __uint_as_float(t.x), v[q + 1] = __uint_as_float(t.y);
+        v[q + 2] = __uint_as_float(t.z), v[q + 3] = __uint_as_float(t.w);
+      } else {
+        v[q] = __hiloint2double(t.y, t.x), v[q + 1] = __hiloint2double(t.w, t.z);
+      }
+    }
+  } else if constexpr (N == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    v[0] = t.x, v[1] = t.y;
+  } else {
+    v[0] = p[0];
   }
 }
 
-// Forward sweep of the pivot blocks of one level.  Tasks are (front, chunk)
-// with the chunks of a front in ascending order, so every chunk waits only
-// on tasks of lower index; the grid is co-resident (cooperative launch) and
-// blocks take tasks from a counter as they come free, so tasks start in
-// ascending order, which rules out a cycle of waits.  Tile s: y_s = Linv_s W[k0:k1]; W[r] -= L[r, k0:k1] y_s, r >= k1.
-// The factor columns and inverse of tile s+1 are staged (double buffer)
-// while tile s waits for its flag and is applied.
+// One pivot-block chunk (rows [c0, c1) of the pivots of front f, columns
+// [r0, r0 + nr) of the pass) of a forward (FWD) or backward sweep, by the
+// DIAG_ROWS threads of a CTA.
+//   forward, tile s: y_s = Linv_s w[k0:k1]; w[r] -= L[r, k0:k1] y_s, r >= k1
+//   backward, tile s (from the last): x_s = Uinv_s w[k0:k1];
+//            w[r] -= U[r, k0:k1] x_s, r < k0
+// init(row, r): the chunk's starting right-hand side; done(row, r, v): what
+// else becomes of a solved element; Yp (leading dimension f.p, column r0
+// first): where tiles are published and waited for.
+//
+// The chain of tiles is bound by the hand-over between CTAs and by shared
+// memory, which serves 128 requested bytes a cycle, broadcasts included.
+// So the chunk's right-hand side stays in registers, a thread holding TR rows
+// x TC columns (4 x 4 at 16 columns: 8 cycles of requests for 16
+// multiply-adds where a row per thread takes 17), and a tile is handed over
+// through its values alone: no fence, flag or second load.  With the
+// products below, 64 columns on a 54^3 grid 20.1 -> 15.6 ms (pivot blocks
+// 9.5 -> 6.5, products 5.8 -> 3.9), 13 FP64 columns on 37^3 2.44 -> 1.66 ms.
+template <typename T, int R, bool FWD, typename Init, typename Done>
+__device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
+                                            const T* __restrict__ F,
+                                            const T* __restrict__ INV,
+                                            int chunk, int nr, T* Yp, T* Ls0,
+                                            T* Xs0, ChunkSmem<T, R>& sm,
+                                            Init init, Done done, int* err) {
+  constexpr int V = 16 / sizeof(T), RS = ChunkSmem<T, R>::RS;
+  constexpr int TC = R >= 4 ? R / 4 : 1, TR = R / TC;  // register tile
+  constexpr int NG = R / TC, NT = DIAG_ROWS / NG;      // column groups, lanes
+  constexpr int VW = TR < V ? TR : V, NP = TR / VW;    // row pieces of VW rows
+  static_assert(NT * TR == DIAG_ROWS, "a chunk is one register tile a thread");
+  const int tid = threadIdx.x, tx = tid % NT, tc = (tid / NT) * TC;
+  const int c0 = chunk * DIAG_ROWS, c1 = min(f.p, c0 + DIAG_ROWS);
+  const int ntiles = (f.p + NB - 1) / NB;
+  // first row (in the chunk) of piece p
+  auto prow = [&](int p) { return (p * NT + tx) * VW; };
+  // stages tile s into buffer s & 1: the rows of this chunk it updates and,
+  // for the chunk that owns it, its inverse
+  auto stage = [&](int s) {
+    const int b = s & 1, k0 = s * NB, kb = min(NB, f.p - k0), k1 = k0 + kb;
+    const T* inv = INV + f.inv_off + (int64_t)s * 2 * NB * NB;
+    if (FWD) {
+      stage_cols(Ls0 + b * NB * DIAG_ROWS, F, f, c0, max(c0, k1) & ~(V - 1), c1,
+                 k0, kb);
+      if (k0 >= c0) stage_inv(Xs0 + b * NB * NB, inv);
+    } else {
+      stage_cols(Ls0 + b * NB * DIAG_ROWS, F, f, c0, c0, min(c1, k0), k0, kb);
+      if (k0 < c1) stage_inv(Xs0 + b * NB * NB, inv + NB * NB);
+    }
+  };
+  // the chunk's tiles: forward from 0 to its last, backward from the last
+  // of the front to its first
+  const int sA = FWD ? 0 : ntiles - 1, sB = FWD ? (c1 - 1) / NB : c0 / NB;
+  const int ds = FWD ? 1 : -1;
+  // two tiles are in flight: what a tile needs is requested a whole tile
+  // before the chunk can use it
+  stage(sA);
+  cp_async_commit();
+  if (sA != sB) stage(sA + ds);
+  cp_async_commit();
+  T w[NP][VW][TC];
+#pragma unroll
+  for (int p = 0; p < NP; p++)
+#pragma unroll
+    for (int a = 0; a < VW; a++)
+#pragma unroll
+      for (int c = 0; c < TC; c++) {
+        const int row = c0 + prow(p) + a, r = tc + c;
+        w[p][a][c] = row < c1 && r < nr ? init(row, r) : (T)0;
+      }
+  for (int s = sA;; s += ds) {
+    const int k0 = s * NB, kb = min(NB, f.p - k0);
+    const bool owner = FWD ? k0 >= c0 : k0 < c1;
+    const T* Ls = Ls0 + (s & 1) * NB * DIAG_ROWS;
+    const T* Xs = Xs0 + (s & 1) * NB * NB;
+    T(*ys)[RS] = sm.ys;
+    if (owner) {
+      // the tile's right-hand side from the registers that hold it
+#pragma unroll
+      for (int p = 0; p < NP; p++) {
+        const int lr = c0 + prow(p) - k0;  // row in the tile
+        if (lr >= 0 && lr < NB)
+#pragma unroll
+          for (int a = 0; a < VW; a++)
+#pragma unroll
+            for (int c = 0; c < TC; c++)
+              sm.ws[lr + a][tc + c] = lr + a < kb ? w[p][a][c] : (T)0;
+      }
+      cp_async_wait_prev();
+      __syncthreads();
+      constexpr int AR = R >= 4 ? 2 : 1;                       // rows
+      constexpr int AC = (NB * R / DIAG_ROWS + AR - 1) / AR;   // x columns
+      constexpr int AL = NB / AR;                              // row lanes
+      const int i0 = (tid % AL) * AR, g0 = (tid / AL) * (AC > 0 ? AC : 1);
+      if (g0 < R) {
+        T acc[AR][AC > 0 ? AC : 1];
+        constexpr int C = AC > 0 ? AC : 1;
+#pragma unroll
+        for (int a = 0; a < AR; a++)
+#pragma unroll
+          for (int c = 0; c < C; c++) acc[a][c] = (T)0;
+        if constexpr (C == 1) {
+          // (few columns: four partial sums shorten the chain of adds)
+          T part[4][AR];
+#pragma unroll
+          for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int a = 0; a < AR; a++) part[q][a] = (T)0;
+#pragma unroll 4
+          for (int m = 0; m < NB; m += 4)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              T xv[AR];
+              lds(Xs + i0 + (m + q) * NB, xv);
+              const T v = sm.ws[m + q][g0];
+#pragma unroll
+              for (int a = 0; a < AR; a++) part[q][a] += xv[a] * v;
+            }
+#pragma unroll
+          for (int a = 0; a < AR; a++)
+            acc[a][0] = (part[0][a] + part[1][a]) + (part[2][a] + part[3][a]);
+        } else {
+#pragma unroll 4
+          for (int m = 0; m < NB; m++) {
+            T xv[AR], v[C];
+            lds(Xs + i0 + m * NB, xv);
+            lds(&sm.ws[m][g0], v);
+#pragma unroll
+            for (int a = 0; a < AR; a++)
+#pragma unroll
+              for (int c = 0; c < C; c++) acc[a][c] += xv[a] * v[c];
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < C; c++)
+#pragma unroll
+          for (int a = 0; a < AR; a++) {
+            const int i = i0 + a, r = g0 + c;
+            const bool in = i < kb && r < nr;
+            ys[i][r] = in ? acc[a][c] : (T)0;
+            if (in) {
+              SweepNan<T>::publish(Yp + k0 + i + (int64_t)r * f.p, acc[a][c]);
+              done(k0 + i, r, acc[a][c]);
+            }
+          }
+      }
+      if (s == sB) break;  // nothing of the chunk is left
+    } else {
+      constexpr int N = (NB * R + DIAG_ROWS - 1) / DIAG_ROWS;
+      T v[N];
+      auto off = [&](int q) -> int64_t {
+        const int e = tid + DIAG_ROWS * q, i = e % NB, r = e / NB;
+        return i < kb && r < nr ? k0 + i + (int64_t)r * f.p : -1;
+      };
+      if (!poll_all<T, N>(Yp, off, v, err)) sm.bad = 1;
+#pragma unroll
+      for (int q = 0; q < N; q++) {
+        const int e = tid + DIAG_ROWS * q, i = e % NB, r = e / NB;
+        if (r < R) ys[i][r] = off(q) >= 0 ? v[q] : (T)0;
+      }
+      cp_async_wait_prev();
+    }
+    __syncthreads();
+    if (sm.bad) return false;
+    // rows [u0, u1) of the chunk take this tile's update
+    const int u0 = FWD ? max(0, k0 + NB - c0) : 0;
+    const int u1 = FWD ? c1 - c0 : min(c1, k0) - c0;
+    bool any = false;
+#pragma unroll
+    for (int p = 0; p < NP; p++) any |= prow(p) >= u0 && prow(p) < u1;
+    if (any) {
+      T acc[NP][VW][TC];
+#pragma unroll
+      for (int p = 0; p < NP; p++)
+#pragma unroll
+        for (int a = 0; a < VW; a++)
+#pragma unroll
+          for (int c = 0; c < TC; c++) acc[p][a][c] = (T)0;
+#pragma unroll 4
+      for (int m = 0; m < kb; m++) {
+        T y[TC];
+        lds(&ys[m][tc], y);
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+          T l[VW];
+          lds(Ls + m * DIAG_ROWS + prow(p), l);
+#pragma unroll
+          for (int a = 0; a < VW; a++)
+#pragma unroll
+            for (int c = 0; c < TC; c++) acc[p][a][c] += l[a] * y[c];
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < NP; p++)
+        if (prow(p) >= u0 && prow(p) < u1)
+#pragma unroll
+          for (int a = 0; a < VW; a++)
+#pragma unroll
+            for (int c = 0; c < TC; c++) w[p][a][c] -= acc[p][a][c];
+    }
+    __syncthreads();  // the tile's buffers are read
+    if (FWD ? s + 2 <= sB : s - 2 >= sB) stage(s + 2 * ds);
+    cp_async_commit();
+  }
+  return true;
+}
+
+// Forward (FWD) or backward sweep of the pivot blocks of one level.  Tasks
+// are (front, chunk) with the chunks of a front in ascending (backward:
+// descending) order, so every chunk waits only on tasks of lower index; the
+// grid is co-resident (cooperative launch) and blocks take tasks from a
+// counter as they come free, so tasks start in ascending order, which rules
+// out a cycle of waits.  The pivot rows of W are dead after the forward
+// sweep (Y carries the result); the backward sweep also writes the final
+// solution to X in original row order.
+template <typename T, int R, bool FWD>
+__device__ __forceinline__ void diag_sweep_body(
+    const SweepTask* __restrict__ tasks, int nbase, int ngroups,
+    const FrontDev* __restrict__ fr, const T* __restrict__ F,
+    const T* __restrict__ INV, int nrhs, const T* __restrict__ W, T* Y,
+    const int* __restrict__ gidx, double* __restrict__ X, int ldx,
+    int* next_task, int* err) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* Ls0 = reinterpret_cast<T*>(smem_raw);  // [2][NB][DIAG_ROWS]
+  T* Xs0 = Ls0 + 2 * NB * DIAG_ROWS;         // [2][NB * NB]
+  __shared__ ChunkSmem<T, R> sm;
+  __shared__ int s_task;
+  if (threadIdx.x == 0) sm.bad = 0;
+  for (;;) {
+    // tasks start in ascending order as blocks come free
+    cp_async_wait_all();
+    __syncthreads();
+    if (threadIdx.x == 0) s_task = atomicAdd(next_task, 1);
+    __syncthreads();
+    const int task = s_task;
+    if (task >= nbase * ngroups) break;
+    // task = group g's copy of base task task - g nbase: columns
+    // [g R, g R + nr) of the pass
+    const int g = task / nbase;
+    const SweepTask t = tasks[task - g * nbase];
+    const int r0 = g * R, nr = min(R, nrhs - r0);
+    const FrontDev f = fr[t.front];
+    const T* Wf = W + f.w_off * nrhs + (int64_t)r0 * (f.p + f.q);
+    T* Yf = Y + f.y_off * nrhs + (int64_t)r0 * f.p;
+    const int dim = f.p + f.q;
+    const int* gi = gidx + f.idx_off;
+    const bool ok = chunk_sweep<T, R, FWD>(
+        f, F, INV, t.chunk, nr, Yf, Ls0, Xs0, sm,
+        [&](int row, int r) { return Wf[row + (int64_t)r * dim]; },
+        [&](int row, int r, T v) {
+          if (!FWD && X) X[gi[row] + (int64_t)(r0 + r) * ldx] = (double)v;
+        },
+        err);
+    if (!ok) break;
+  }
+  cp_async_wait_all();
+}
+
 template <typename T, int R>
 __global__ void __launch_bounds__(DIAG_ROWS)
     k_fwd_diag(const SweepTask* __restrict__ tasks, int nbase, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
-               const T* __restrict__ INV, const int64_t* __restrict__ flag_off,
-               int64_t gstride, int nrhs, T* __restrict__ W,
-               T* __restrict__ Y, const int* __restrict__ gidx,
-               double* __restrict__ X, int ldx, int* flags, int* next_task,
-               int* err) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* Ls0 = reinterpret_cast<T*>(smem_raw);  // [2][NB][DIAG_ROWS]
-  T* Xs0 = Ls0 + 2 * NB * DIAG_ROWS;         // [2][NB * NB]
-  __shared__ T ws[NB][R];
-  __shared__ T ys[NB][R];
-  __shared__ T Wc[R][DIAG_ROWS];  // this chunk's rows of W (its group's columns)
-  __shared__ int bad, s_task;
-  const int tid = threadIdx.x;
-  constexpr int V = 16 / sizeof(T);
-  if (tid == 0) bad = 0;
-  for (;;) {
-    // tasks start in ascending order as blocks come free
-    __syncthreads();
-    if (tid == 0) s_task = atomicAdd(next_task, 1);
-    __syncthreads();
-    const int task = s_task;
-    if (task >= nbase * ngroups) break;
-    // task = group g's copy of base task task - g nbase: columns
-    // [g R, g R + nr) of the pass, with the group's own tile flags
-    const int g = task / nbase;
-    const SweepTask t = tasks[task - g * nbase];
-    const int r0 = g * R, nr = min(R, nrhs - r0);
-    const FrontDev f = fr[t.front];
-    const int dim = f.p + f.q;
-    const int c0 = t.chunk * DIAG_ROWS, c1 = min(f.p, c0 + DIAG_ROWS);
-    const int ntiles = (f.p + NB - 1) / NB;
-    int* fl = flags + g * gstride + flag_off[t.front];
-    T* Wf = W + f.w_off * nrhs;
-    T* Yf = Y + f.y_off * nrhs;
-    const int row = c0 + tid;
-    // stages tile s into buffer b: the rows of this chunk it updates and,
-    // for the chunk that owns it, its inverse
-    auto stage = [&](int s, int b) {
-      const int k0 = s * NB, kb = min(NB, f.p - k0), k1 = k0 + kb;
-      const int u0 = max(c0, k1);
-      stage_cols(Ls0 + b * NB * DIAG_ROWS, F, f, c0, u0 & ~(V - 1), c1, k0, kb);
-      if (k0 >= c0)
-        stage_inv(Xs0 + b * NB * NB, INV + f.inv_off + (int64_t)s * 2 * NB * NB);
-    };
-    cp_async_wait_all();
-    __syncthreads();
-    stage(0, 0);
-    cp_async_commit();
-    // the pivot rows of W are dead after this sweep (Y carries the result),
-    // so the chunk keeps its rows in shared memory and never writes them back
-#pragma unroll
-    for (int r = 0; r < R; r++)
-      Wc[r][tid] =
-          (row < c1 && r < nr) ? Wf[row + (int64_t)(r0 + r) * dim] : (T)0;
-    for (int s = 0; s < ntiles; s++) {
-      const int k0 = s * NB, kb = min(NB, f.p - k0), k1 = k0 + kb;
-      if (k0 >= c1) break;  // owned by a later chunk; updates no row of ours
-      const bool owner = k0 >= c0;
-      const int u0 = max(c0, k1);  // rows [u0, c1) take this tile's update
-      const T* Ls = Ls0 + (s & 1) * NB * DIAG_ROWS;
-      const T* Xs = Xs0 + (s & 1) * NB * NB;
-      if (s + 1 < ntiles && (s + 1) * NB < c1) stage(s + 1, (s + 1) & 1);
-      cp_async_commit();
-      if (!owner && tid == 0 && !wait_flag(fl + s, err)) bad = 1;
-      cp_async_wait_prev();  // tile s staged (tile s+1 may still be in flight)
-      __syncthreads();
-      if (bad) return;
-      {
-        if (owner) {
-          for (int e = tid; e < NB * R; e += blockDim.x) {
-            const int i = e % NB, r = e / NB;
-            ws[i][r] = (i < kb && r < nr) ? Wc[r][k0 - c0 + i] : (T)0;
-          }
-          __syncthreads();
-          tile_apply<T, R>(Xs, ws, ys, Yf, f.p, k0, kb, r0, nr);
-          __syncthreads();  // raise_flag's fence publishes the CTA's Y stores
-          if (tid == 0) raise_flag(fl + s);
-        } else {
-          for (int e = tid; e < NB * R; e += blockDim.x) {
-            const int i = e % NB, r = e / NB;
-            ys[i][r] = (i < kb && r < nr)
-                           ? __ldcg(Yf + k0 + i + (int64_t)(r0 + r) * f.p)
-                           : (T)0;
-          }
-          __syncthreads();
-        }
-        if (row >= u0 && row < c1) {
-          T acc[R];
-#pragma unroll
-          for (int r = 0; r < R; r++) acc[r] = (T)0;
-#pragma unroll 8
-          for (int m = 0; m < kb; m++) {
-            const T l = Ls[m * DIAG_ROWS + tid];
-#pragma unroll
-            for (int r = 0; r < R; r++) acc[r] += l * ys[m][r];
-          }
-#pragma unroll
-          for (int r = 0; r < R; r++)
-            if (r < nr) Wc[r][tid] -= acc[r];
-        }
-        __syncthreads();
-      }
-    }
-  }
-  cp_async_wait_all();
+               const T* __restrict__ INV, int nrhs, const T* __restrict__ W,
+               T* Y, const int* __restrict__ gidx, double* __restrict__ X,
+               int ldx, int* next_task, int* err) {
+  diag_sweep_body<T, R, true>(tasks, nbase, ngroups, fr, F, INV, nrhs, W, Y,
+                              gidx, X, ldx, next_task, err);
 }
 
-// Backward sweep of the pivot blocks of one level (after W[0:p] -= U12 x_Q).
-// Tasks list the chunks of a front from the last to the first, so again
-// every wait is on a task of lower index.  Tile s (from the last):
-// x_s = Uinv_s W[k0:k1]; W[r] -= U[r, k0:k1] x_s for r < k0.  Staging of
-// tile s-1 overlaps tile s as in the forward sweep.
 template <typename T, int R>
 __global__ void __launch_bounds__(DIAG_ROWS)
     k_bwd_diag(const SweepTask* __restrict__ tasks, int nbase, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
-               const T* __restrict__ INV, const int64_t* __restrict__ flag_off,
-               int64_t gstride, int nrhs, T* __restrict__ W,
-               T* __restrict__ Y, const int* __restrict__ gidx,
-               double* __restrict__ X, int ldx, int* flags, int* next_task,
-               int* err) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* Ls0 = reinterpret_cast<T*>(smem_raw);
-  T* Xs0 = Ls0 + 2 * NB * DIAG_ROWS;
-  __shared__ T ws[NB][R];
-  __shared__ T xs[NB][R];
-  __shared__ T Wc[R][DIAG_ROWS];  // this chunk's rows of W (its group's columns)
-  __shared__ int bad, s_task;
-  const int tid = threadIdx.x;
-  if (tid == 0) bad = 0;
-  for (;;) {
-    __syncthreads();
-    if (tid == 0) s_task = atomicAdd(next_task, 1);
-    __syncthreads();
-    const int task = s_task;
-    if (task >= nbase * ngroups) break;
-    // task = group g's copy of base task task - g nbase: columns
-    // [g R, g R + nr) of the pass, with the group's own tile flags
-    const int g = task / nbase;
-    const SweepTask t = tasks[task - g * nbase];
-    const int r0 = g * R, nr = min(R, nrhs - r0);
-    const FrontDev f = fr[t.front];
-    const int dim = f.p + f.q;
-    const int c0 = t.chunk * DIAG_ROWS, c1 = min(f.p, c0 + DIAG_ROWS);
-    const int ntiles = (f.p + NB - 1) / NB;
-    int* fl = flags + g * gstride + flag_off[t.front];
-    T* Wf = W + f.w_off * nrhs;
-    T* Yf = Y + f.y_off * nrhs;
-    const int row = c0 + tid;
-    auto stage = [&](int s, int b) {
-      const int k0 = s * NB, kb = min(NB, f.p - k0);
-      stage_cols(Ls0 + b * NB * DIAG_ROWS, F, f, c0, c0, min(c1, k0), k0, kb);
-      if (k0 < c1)
-        stage_inv(Xs0 + b * NB * NB,
-                  INV + f.inv_off + (int64_t)s * 2 * NB * NB + NB * NB);
-    };
-    cp_async_wait_all();
-    __syncthreads();
-    stage(ntiles - 1, (ntiles - 1) & 1);
-    cp_async_commit();
-#pragma unroll
-    for (int r = 0; r < R; r++)
-      Wc[r][tid] =
-          (row < c1 && r < nr) ? Wf[row + (int64_t)(r0 + r) * dim] : (T)0;
-    for (int s = ntiles - 1; s >= 0; s--) {
-      const int k0 = s * NB, kb = min(NB, f.p - k0);
-      if (k0 < c0) break;  // tile lies above our rows: nothing left
-      const bool owner = k0 < c1;
-      const int u1 = min(c1, k0);  // rows [c0, u1) take this tile's update
-      const T* Ls = Ls0 + (s & 1) * NB * DIAG_ROWS;
-      const T* Xs = Xs0 + (s & 1) * NB * NB;
-      if (s >= 1 && (s - 1) * NB >= c0) stage(s - 1, (s - 1) & 1);
-      cp_async_commit();
-      if (!owner && tid == 0 && !wait_flag(fl + s, err)) bad = 1;
-      cp_async_wait_prev();
-      __syncthreads();
-      if (bad) return;
-      {
-        if (owner) {
-          for (int e = tid; e < NB * R; e += blockDim.x) {
-            const int i = e % NB, r = e / NB;
-            ws[i][r] = (i < kb && r < nr) ? Wc[r][k0 - c0 + i] : (T)0;
-          }
-          __syncthreads();
-          tile_apply<T, R>(Xs, ws, xs, Yf, f.p, k0, kb, r0, nr);
-          __syncthreads();
-          if (tid == 0) raise_flag(fl + s);
-          if (X) {  // the tile's final solution also into X (original rows)
-            const int* g = gidx + f.idx_off;
-            for (int e = tid; e < NB * R; e += blockDim.x) {
-              const int i = e % NB, r = e / NB;
-              if (i < kb && r < nr)
-                X[g[k0 + i] + (int64_t)(r0 + r) * ldx] = (double)xs[i][r];
-            }
-          }
-        } else {
-          for (int e = tid; e < NB * R; e += blockDim.x) {
-            const int i = e % NB, r = e / NB;
-            xs[i][r] = (i < kb && r < nr)
-                           ? __ldcg(Yf + k0 + i + (int64_t)(r0 + r) * f.p)
-                           : (T)0;
-          }
-          __syncthreads();
-        }
-        if (row < u1) {
-          T acc[R];
-#pragma unroll
-          for (int r = 0; r < R; r++) acc[r] = (T)0;
-#pragma unroll 8
-          for (int m = 0; m < kb; m++) {
-            const T u = Ls[m * DIAG_ROWS + tid];
-#pragma unroll
-            for (int r = 0; r < R; r++) acc[r] += u * xs[m][r];
-          }
-#pragma unroll
-          for (int r = 0; r < R; r++)
-            if (r < nr) Wc[r][tid] -= acc[r];
-        }
-        __syncthreads();
-      }
-    }
-  }
-  cp_async_wait_all();
+               const T* __restrict__ INV, int nrhs, const T* __restrict__ W,
+               T* Y, const int* __restrict__ gidx, double* __restrict__ X,
+               int ldx, int* next_task, int* err) {
+  diag_sweep_body<T, R, false>(tasks, nbase, ngroups, fr, F, INV, nrhs, W, Y,
+                               gidx, X, ldx, next_task, err);
 }
 
-// Backward start of a front: W[0:p] = Y (the forward result) and
-// W[p:dim] = X[gidx] (the non-pivot solution, already final).
+// Backward start of a front: W[0:p] = Y (the forward result; Y is marked
+// unsolved again for the backward sweep) and W[p:dim] = X[gidx] (the
+// non-pivot solution, already final).
 template <typename T>
 __global__ void k_bwd_init(const int* __restrict__ list,
                            const FrontDev* __restrict__ fr,
                            const int* __restrict__ gidx,
                            const double* __restrict__ X, int ldx, int nrhs,
-                           const T* __restrict__ Y, T* __restrict__ W) {
+                           T* __restrict__ Y, T* __restrict__ W) {
   const FrontDev f = fr[list[blockIdx.x / SOLVE_SPLIT]];
   const int dim = f.p + f.q;
   T* w = W + f.w_off * nrhs;
-  const T* y = Y + f.y_off * nrhs;
+  T* y = Y + f.y_off * nrhs;
   const int* g = gidx + f.idx_off;
   // one row per thread (its index once), all right-hand sides
   for (int t = (blockIdx.x % SOLVE_SPLIT) * blockDim.x + threadIdx.x; t < dim;
        t += SOLVE_SPLIT * blockDim.x) {
     if (t < f.p) {
-      for (int r = 0; r < nrhs; r++)
+      for (int r = 0; r < nrhs; r++) {
         w[t + (int64_t)r * dim] = y[t + (int64_t)r * f.p];
+        y[t + (int64_t)r * f.p] = SweepNan<T>::mark();
+      }
     } else {
       const int64_t gt = g[t];
       for (int r = 0; r < nrhs; r++)
@@ -407,99 +510,128 @@ constexpr int GEMV_ROWS = 64, GEMV_K = 256;
 // writer (the bit-reproducible schedule).
 //   FWD:  W[p + i] -= L21[i, :] Y        (i < q, over the p pivot columns)
 //   !FWD: W[i]     -= U12[i, :] W[p:dim] (i < p, over the q update columns)
-// Blocks [g ntasks, (g + 1) ntasks) take columns [g R, g R + R) of the
-// pass (R >= nrhs: one group, every column).
+// Blocks of one task are neighbours (they share its factor entries in L2)
+// and take columns [g R, g R + R) of the pass each.
+//
+// A lane holds two rows (one value of the vector slice, which shared memory
+// broadcasts at one requested word a cycle, serves two multiply-adds), a
+// warp an eighth of the columns; GEMV_LD of its factor entries are in
+// flight at a time, the first of them before the slice is staged.
 template <typename T, int R, bool FWD>
 __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
-                                         int ntasks,
+                                         int ngroups,
                                          const FrontDev* __restrict__ fr,
                                          const T* __restrict__ F, int nrhs,
                                          T* __restrict__ W,
                                          const T* __restrict__ Y) {
+  constexpr int RS = ChunkSmem<T, R>::RS;
+  constexpr int KW = GEMV_K / 8;  // columns per warp
+  constexpr int UB = R <= 4 ? 16 : 8;  // columns in flight (two rows each)
   // the block's slice of the source vector, then (after the products) the
-  // reduction of the four k-groups, in one buffer
-  constexpr size_t YS = sizeof(T) * GEMV_K * R,
+  // partial sums of four warps, in one buffer
+  constexpr size_t YS = sizeof(T) * GEMV_K * RS,
                    RED = sizeof(T) * 4 * GEMV_ROWS * (R + 1);
   __shared__ __align__(16) unsigned char smb[YS > RED ? YS : RED];
-  T(*ys)[R] = reinterpret_cast<T(*)[R]>(smb);
+  T(*ys)[RS] = reinterpret_cast<T(*)[RS]>(smb);
   T(*red)[GEMV_ROWS][R + 1] = reinterpret_cast<T(*)[GEMV_ROWS][R + 1]>(smb);
-  const int cg = blockIdx.x / ntasks;  // column group
-  const SweepTask t = tasks[blockIdx.x - cg * ntasks];
+  const SweepTask t = tasks[blockIdx.x / ngroups];
+  const int r0 = (blockIdx.x % ngroups) * R, nr = min(R, nrhs - r0);
   const FrontDev f = fr[t.front];
   const int dim = f.p + f.q;
   const int nrows = FWD ? f.q : f.p, nk = FWD ? f.p : f.q;
-  const int i = t.chunk * GEMV_ROWS + (threadIdx.x & 63), g = threadIdx.x >> 6;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i0 = t.chunk * GEMV_ROWS + lane;  // rows i0 and i0 + 32
   const int nkb = (nk + GEMV_K - 1) / GEMV_K;
   const int kb0 = t.kchunk < 0 ? 0 : t.kchunk,
             kb1 = t.kchunk < 0 ? nkb : t.kchunk + 1;
-  T* Wf = W + f.w_off * nrhs;
+  T* Wf = W + f.w_off * nrhs + (int64_t)r0 * dim;
   // source vector (ld lds) and the operand block's first element
-  const T* src = FWD ? Y + f.y_off * nrhs : Wf + f.p;
-  const int lds = FWD ? f.p : dim;
-  const T* a = FWD ? F + f.off + f.p + i : F + f.off + i + (int64_t)f.p * f.ld;
+  const T* src = FWD ? Y + f.y_off * nrhs + (int64_t)r0 * f.p : Wf + f.p;
+  const int lds_ = FWD ? f.p : dim;
+  const T* a = FWD ? F + f.off + f.p + i0 : F + f.off + i0 + (int64_t)f.p * f.ld;
   T* dst = FWD ? Wf + f.p : Wf;
-  for (int r0 = cg * R; r0 < min(nrhs, cg * R + R); r0 += R) {
-    const int nr = min(R, nrhs - r0);
-    T acc[R];
+  const bool in0 = i0 < nrows, in1 = i0 + 32 < nrows;
+  T acc[2][R];
 #pragma unroll
-    for (int r = 0; r < R; r++) acc[r] = (T)0;
-    for (int kb = kb0; kb < kb1; kb++) {
-      const int kc0 = kb * GEMV_K, kc1 = min(nk, kc0 + GEMV_K);
-      __syncthreads();  // the previous pass's ys / reduction is read
-      for (int e = threadIdx.x; e < GEMV_K * R; e += blockDim.x) {
-        const int k = e % GEMV_K, r = e / GEMV_K;
-        ys[k][r] = (kc0 + k < kc1 && r < nr)
-                       ? src[kc0 + k + (int64_t)(r0 + r) * lds]
-                       : (T)0;
+  for (int r = 0; r < R; r++) acc[0][r] = acc[1][r] = (T)0;
+  for (int kb = kb0; kb < kb1; kb++) {
+    const int kc0 = kb * GEMV_K, kc1 = min(nk, kc0 + GEMV_K);
+    const int w0 = kc0 + warp * KW;
+    T av[UB][2];
+    auto load = [&](int k0) {
+#pragma unroll
+      for (int u = 0; u < UB; u++) {
+        const bool ink = k0 + u < kc1;
+        av[u][0] = ink && in0 ? a[(int64_t)(k0 + u) * f.ld] : (T)0;
+        av[u][1] = ink && in1 ? a[(int64_t)(k0 + u) * f.ld + 32] : (T)0;
       }
-      __syncthreads();
-      if (i < nrows) {
-        constexpr int UB = R <= 4 ? 8 : (R <= 8 ? 4 : 2);  // loads in flight
-        for (int k0 = kc0 + g; k0 < kc1; k0 += 4 * UB) {
-          T av[UB], wv[UB][R];
+    };
+    load(w0);
+    if (kb > kb0) __syncthreads();  // the previous block's slice is read
 #pragma unroll
-          for (int u = 0; u < UB; u++) {
-            const int k = k0 + 4 * u;
-            av[u] = k < kc1 ? a[(int64_t)k * f.ld] : (T)0;
+    for (int r = 0; r < R; r++) {
+      const int k = threadIdx.x;
+      ys[k][r] = kc0 + k < kc1 && r < nr ? src[kc0 + k + (int64_t)r * lds_] : (T)0;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k0 = 0; k0 < KW; k0 += UB) {
+      if (w0 + k0 >= kc1) break;
+      if (k0) load(w0 + k0);
 #pragma unroll
-            for (int r = 0; r < R; r++) wv[u][r] = ys[min(k, kc1 - 1) - kc0][r];
-          }
+      for (int u = 0; u < UB; u++) {
+        T y[R];
+        lds(ys[warp * KW + k0 + u], y);
 #pragma unroll
-          for (int u = 0; u < UB; u++)
-#pragma unroll
-            for (int r = 0; r < R; r++) acc[r] += av[u] * wv[u][r];
+        for (int r = 0; r < R; r++) {
+          acc[0][r] += av[u][0] * y[r];
+          acc[1][r] += av[u][1] * y[r];
         }
       }
     }
-    __syncthreads();  // ys is read
+  }
+  __syncthreads();  // ys is read
+  // eight partial sums per row: warps 4-7 hand theirs to warps 0-3, those
+  // four are then added up by all threads
+  if (warp >= 4) {
 #pragma unroll
-    for (int r = 0; r < R; r++) red[g][threadIdx.x & 63][r] = acc[r];
-    __syncthreads();
-    if (g == 0 && i < nrows) {
-      for (int r = 0; r < nr; r++) {
-        T s = red[0][threadIdx.x][r] + red[1][threadIdx.x][r] +
-              red[2][threadIdx.x][r] + red[3][threadIdx.x][r];
-        atomicAdd(dst + i + (int64_t)(r0 + r) * dim, -s);
-      }
+    for (int r = 0; r < R; r++) {
+      red[warp - 4][lane][r] = acc[0][r];
+      red[warp - 4][lane + 32][r] = acc[1][r];
     }
-    __syncthreads();
+  }
+  __syncthreads();
+  if (warp < 4) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      red[warp][lane][r] += acc[0][r];
+      red[warp][lane + 32][r] += acc[1][r];
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < GEMV_ROWS * R; e += 256) {
+    const int i = e % GEMV_ROWS, r = e / GEMV_ROWS;
+    if (t.chunk * GEMV_ROWS + i < nrows && r < nr) {
+      const T s = (red[0][i][r] + red[1][i][r]) + (red[2][i][r] + red[3][i][r]);
+      atomicAdd(dst + t.chunk * GEMV_ROWS + i + (int64_t)r * dim, -s);
+    }
   }
 }
 
 template <typename T, int R>
 __global__ void __launch_bounds__(256)
-    k_gemv_l21(const SweepTask* __restrict__ tasks, int ntasks,
+    k_gemv_l21(const SweepTask* __restrict__ tasks, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
                int nrhs, T* __restrict__ W, const T* __restrict__ Y) {
-  gemv_off<T, R, true>(tasks, ntasks, fr, F, nrhs, W, Y);
+  gemv_off<T, R, true>(tasks, ngroups, fr, F, nrhs, W, Y);
 }
 
 template <typename T, int R>
 __global__ void __launch_bounds__(256)
-    k_gemv_u12(const SweepTask* __restrict__ tasks, int ntasks,
+    k_gemv_u12(const SweepTask* __restrict__ tasks, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
                int nrhs, T* __restrict__ W, const T* __restrict__ Y) {
-  gemv_off<T, R, false>(tasks, ntasks, fr, F, nrhs, W, Y);
+  gemv_off<T, R, false>(tasks, ngroups, fr, F, nrhs, W, Y);
 }
 
 }  // namespace snu

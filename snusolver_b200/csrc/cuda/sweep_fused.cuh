@@ -10,9 +10,9 @@
 // * forward: Z (n x nrhs, indexed by original row, precision T) starts as B.
 //   Pivot-block chunk task (f, c): waits until every off-diagonal task of
 //   f's children has finished, gathers its rows of Z, solves the tile chain
-//   of f's pivot block (tile flags between the chunks of f, as in
-//   k_fwd_diag) and writes Y_f.  Off-diagonal task (f, 64-row block,
-//   256-column block): waits for the tile flags of its columns, then
+//   of f's pivot block (chunk_sweep: the chunks of f hand tiles over through
+//   Y_f) and writes Y_f.  Off-diagonal task (f, 64-row block, 256-column
+//   block): waits for its columns of Y_f, then
 //   Z[gidx[p + i]] -= L21[i, :] Y_f with atomics -- straight into the rows
 //   of whichever ancestor pivots them (no extend-add: the elimination tree
 //   guarantees only f's descendants update f's pivot rows).
@@ -21,7 +21,9 @@
 //   block (then every ancestor has), reads x_Q from X (FP64) and
 //   Y_f[i] -= U12[i, :] x_Q with atomics.  Pivot-block chunk task: waits for
 //   all of f's off-diagonal tasks, solves the chain with the tile inverses
-//   (descending), writes x_P to Y_f and to X[gidx[...]] (FP64).
+//   (descending), writes x_P to X[gidx[...]] (FP64) and hands tiles over
+//   through Z, which the forward sweep is done with (marked unsolved again
+//   between the sweeps).
 //
 // A front's "children" here are its nearest descendants with pivots (fronts
 // without pivots pass their rows on; dep.effpar skips them).  Tasks are
@@ -58,14 +60,20 @@ struct SweepDep {
 __device__ __forceinline__ bool wait_count(const int* ctr, int target,
                                            int* err) {
   for (long it = 0; it < WAVE_SPIN_LIMIT; it++) {
-    if (*(const volatile int*)ctr >= target) {
-      __threadfence();
-      return true;
-    }
-    __nanosleep(64);
+    int v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(ctr)
+                 : "memory");
+    if (v >= target) return true;
+    if (it > 4) __nanosleep(20);
   }
   atomicExch(err, 1);
   return false;
+}
+
+// Adds one to a counter, with a release at GPU scope (by one thread after
+// the CTA barrier that follows the CTA's writes, as raise_flag).
+__device__ __forceinline__ void count_one(int* ctr) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(ctr) : "memory");
 }
 
 // Dynamic shared memory: the pivot-block part's staging (two buffers of
@@ -82,7 +90,7 @@ template <typename T, int R, bool FWD>
 __device__ __forceinline__ void fused_offdiag(
     const FrontDev& f, const T* __restrict__ F, const int* __restrict__ g,
     int blk, int kblk, int nrhs, T* Z, int n, T* Yf, const double* X,
-    int ldx, unsigned char* sm) {
+    int ldx, unsigned char* sm, int* err) {
   constexpr size_t YS = sizeof(T) * GEMV_K * R;
   T(*ys)[R] = reinterpret_cast<T(*)[R]>(sm);
   T(*red)[GEMV_ROWS][R + 1] = reinterpret_cast<T(*)[GEMV_ROWS][R + 1]>(sm + YS);
@@ -93,16 +101,31 @@ __device__ __forceinline__ void fused_offdiag(
   for (int r0 = 0; r0 < nrhs; r0 += R) {
     const int nr = min(R, nrhs - r0);
     __syncthreads();  // the previous pass's reduction is read
-    for (int e = threadIdx.x; e < GEMV_K * R; e += blockDim.x) {
-      const int k = e % GEMV_K, r = e / GEMV_K;
-      T v = (T)0;
-      if (kc0 + k < kc1 && r < nr) {
-        if (FWD)  // written by this launch's pivot chunks: through L2
-          v = __ldcg(Yf + kc0 + k + (int64_t)(r0 + r) * f.p);
-        else
-          v = (T)__ldcg(X + g[f.p + kc0 + k] + (int64_t)(r0 + r) * ldx);
+    if (FWD) {  // published by this launch's pivot chunks
+      constexpr int N = GEMV_K * R / DIAG_ROWS, U = N < 8 ? N : 8;
+#pragma unroll 1
+      for (int q0 = 0; q0 < N; q0 += U) {
+        T v[U];
+        auto off = [&](int q) -> int64_t {
+          const int e = threadIdx.x + DIAG_ROWS * (q0 + q), k = e % GEMV_K,
+                    r = e / GEMV_K;
+          return kc0 + k < kc1 && r < nr ? kc0 + k + (int64_t)(r0 + r) * f.p : -1;
+        };
+        // (a timeout is in *err; the values are then as good as any)
+        poll_all<T, U>(Yf, off, v, err);
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+          const int e = threadIdx.x + DIAG_ROWS * (q0 + q);
+          ys[e % GEMV_K][e / GEMV_K] = off(q) >= 0 ? v[q] : (T)0;
+        }
       }
-      ys[k][r] = v;
+    } else {
+      for (int e = threadIdx.x; e < GEMV_K * R; e += blockDim.x) {
+        const int k = e % GEMV_K, r = e / GEMV_K;
+        ys[k][r] = kc0 + k < kc1 && r < nr
+                       ? (T)__ldcg(X + g[f.p + kc0 + k] + (int64_t)(r0 + r) * ldx)
+                       : (T)0;
+      }
     }
     __syncthreads();
     T acc[R];
@@ -146,21 +169,18 @@ __global__ void __launch_bounds__(DIAG_ROWS)
                   const FrontDev* __restrict__ fr,
                   const SweepDep* __restrict__ dep,
                   const int* __restrict__ gidx, const T* __restrict__ F,
-                  const T* __restrict__ INV,
-                  const int64_t* __restrict__ flag_off, int nfronts, int nrhs,
-                  int n, T* Z, T* __restrict__ Y, double* X, int ldx,
-                  int* flags, int* ctr, int* next_task, int* err) {
+                  const T* __restrict__ INV, int nfronts, int nrhs, int n,
+                  T* Z, T* Y, double* X, int ldx, int* ctr, int* next_task,
+                  int* err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Ls0 = reinterpret_cast<T*>(smem_raw);  // [2][NB][DIAG_ROWS]
   T* Xs0 = Ls0 + 2 * NB * DIAG_ROWS;         // [2][NB * NB]
-  __shared__ T ws[NB][R];
-  __shared__ T ys[NB][R];
-  __shared__ T Wc[R][DIAG_ROWS];  // this chunk's rows (nrhs <= R)
-  __shared__ int bad, s_task;
+  __shared__ ChunkSmem<T, R> sm;
+  __shared__ int s_task;
   const int tid = threadIdx.x;
-  constexpr int V = 16 / sizeof(T);
-  if (tid == 0) bad = 0;
+  if (tid == 0) sm.bad = 0;
   for (;;) {
+    cp_async_wait_all();  // (the staging buffers: the next task's, or scratch)
     __syncthreads();
     if (tid == 0) s_task = atomicAdd(next_task, 1);
     __syncthreads();
@@ -170,144 +190,52 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     const FrontDev f = fr[t.front];
     const SweepDep d = dep[t.front];
     const int* g = gidx + f.idx_off;
-    int* fl = flags + flag_off[t.front];
     T* Yf = Y + f.y_off * nrhs;
     if (t.kind == 1) {
       // ------------------------------------------ off-diagonal block
-      cp_async_wait_all();  // (the staging buffers become its scratch)
-      if (tid == 0) {
-        bool ok = true;
-        if (FWD) {  // the pivot tiles of its columns
-          const int s0 = t.b * GEMV_K / NB;
-          const int s1 = (min(f.p, (t.b + 1) * GEMV_K) + NB - 1) / NB;
-          for (int s = s0; s < s1 && ok; s++) ok = wait_flag(fl + s, err);
-        } else if (d.effpar >= 0) {  // the ancestors' x is final
-          ok = wait_count(ctr + 2 * nfronts + d.effpar, dep[d.effpar].nch, err);
-        }
-        if (!ok) bad = 1;
+      if (!FWD) {  // the ancestors' x is final
+        if (tid == 0 && d.effpar >= 0 &&
+            !wait_count(ctr + 2 * nfronts + d.effpar, dep[d.effpar].nch, err))
+          sm.bad = 1;
+        __syncthreads();
+        if (sm.bad) return;
       }
-      __syncthreads();
-      if (bad) return;
       fused_offdiag<T, R, FWD>(f, F, g, t.a, t.b, nrhs, Z, n, Yf, X, ldx,
-                               smem_raw);
-      // every thread's atomics are performed before the count is raised
-      __threadfence();
+                               smem_raw, err);
       __syncthreads();
-      if (tid == 0) {
-        if (FWD) {
-          if (d.effpar >= 0) atomicAdd(ctr + d.effpar, 1);
-        } else {
-          atomicAdd(ctr + nfronts + t.front, 1);
-        }
+      if (tid == 0) {  // (the release orders the CTA's atomics before it)
+        if (!FWD)
+          count_one(ctr + nfronts + t.front);
+        else if (d.effpar >= 0)
+          count_one(ctr + d.effpar);
       }
       continue;
     }
     // ------------------------------------------------ pivot-block chunk
-    const int c0 = t.a * DIAG_ROWS, c1 = min(f.p, c0 + DIAG_ROWS);
-    const int ntiles = (f.p + NB - 1) / NB;
-    const int row = c0 + tid;
     if (tid == 0) {
       const bool ok = FWD ? wait_count(ctr + t.front, d.need, err)
                           : wait_count(ctr + nfronts + t.front, d.ngq, err);
-      if (!ok) bad = 1;
+      if (!ok) sm.bad = 1;
     }
     __syncthreads();
-    if (bad) return;
-    auto stage = [&](int s, int b) {
-      const int k0 = s * NB, kb = min(NB, f.p - k0), k1 = k0 + kb;
-      if (FWD) {
-        const int u0 = max(c0, k1);
-        stage_cols(Ls0 + b * NB * DIAG_ROWS, F, f, c0, u0 & ~(V - 1), c1, k0, kb);
-        if (k0 >= c0)
-          stage_inv(Xs0 + b * NB * NB, INV + f.inv_off + (int64_t)s * 2 * NB * NB);
-      } else {
-        stage_cols(Ls0 + b * NB * DIAG_ROWS, F, f, c0, c0, min(c1, k0), k0, kb);
-        if (k0 < c1)
-          stage_inv(Xs0 + b * NB * NB,
-                    INV + f.inv_off + (int64_t)s * 2 * NB * NB + NB * NB);
-      }
-    };
-    cp_async_wait_all();
-    __syncthreads();
-    const int sfirst = FWD ? 0 : ntiles - 1;
-    stage(sfirst, sfirst & 1);
-    cp_async_commit();
+    if (sm.bad) return;
     // the chunk's rows: forward from Z (gathered), backward from Y_f (the
     // forward result less U12 x_Q); both written by this launch: via L2
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      T v = (T)0;
-      if (row < c1 && r < nrhs)
-        v = FWD ? __ldcg(Z + g[row] + (int64_t)r * n)
-                : __ldcg(Yf + row + (int64_t)r * f.p);
-      Wc[r][tid] = v;
-    }
-    for (int step = 0; step < ntiles; step++) {
-      const int s = FWD ? step : ntiles - 1 - step;
-      const int k0 = s * NB, kb = min(NB, f.p - k0), k1 = k0 + kb;
-      if (FWD ? k0 >= c1 : k0 < c0) break;  // no row of ours left
-      const bool owner = FWD ? k0 >= c0 : k0 < c1;
-      // rows that take this tile's update: forward [max(c0, k1), c1),
-      // backward [c0, min(c1, k0))
-      const int u0 = FWD ? max(c0, k1) : c0, u1 = FWD ? c1 : min(c1, k0);
-      const T* Ls = Ls0 + (s & 1) * NB * DIAG_ROWS;
-      const T* Xs = Xs0 + (s & 1) * NB * NB;
-      const int sn = FWD ? s + 1 : s - 1;
-      if (FWD ? (sn < ntiles && sn * NB < c1) : (sn >= 0 && sn * NB >= c0))
-        stage(sn, sn & 1);
-      cp_async_commit();
-      if (!owner && tid == 0 && !wait_flag(fl + s, err)) bad = 1;
-      cp_async_wait_prev();
-      __syncthreads();
-      if (bad) return;
-      for (int r0 = 0; r0 < nrhs; r0 += R) {
-        const int nr = min(R, nrhs - r0);
-        if (owner) {
-          for (int e = tid; e < NB * R; e += blockDim.x) {
-            const int i = e % NB, r = e / NB;
-            ws[i][r] = (i < kb && r < nr) ? Wc[r0 + r][k0 - c0 + i] : (T)0;
-          }
-          __syncthreads();
-          tile_apply<T, R>(Xs, ws, ys, Yf, f.p, k0, kb, r0, nr);
-          if (!FWD)  // the final solution of these pivots
-            for (int e = tid; e < NB * R; e += blockDim.x) {
-              const int i = e % NB, r = e / NB;
-              if (i < kb && r < nr)
-                X[g[k0 + i] + (int64_t)(r0 + r) * ldx] = (double)ys[i][r];
-            }
-          __syncthreads();  // raise_flag's fence publishes the CTA's stores
-          if (tid == 0 && r0 + R >= nrhs) raise_flag(fl + s);
-        } else {
-          for (int e = tid; e < NB * R; e += blockDim.x) {
-            const int i = e % NB, r = e / NB;
-            ys[i][r] = (i < kb && r < nr)
-                           ? __ldcg(Yf + k0 + i + (int64_t)(r0 + r) * f.p)
-                           : (T)0;
-          }
-          __syncthreads();
-        }
-        if (row >= u0 && row < u1) {
-          T acc[R];
-#pragma unroll
-          for (int r = 0; r < R; r++) acc[r] = (T)0;
-#pragma unroll 8
-          for (int m = 0; m < kb; m++) {
-            const T l = Ls[m * DIAG_ROWS + tid];
-#pragma unroll
-            for (int r = 0; r < R; r++) acc[r] += l * ys[m][r];
-          }
-#pragma unroll
-          for (int r = 0; r < R; r++)
-            if (r < nr) Wc[r0 + r][tid] -= acc[r];
-        }
-        __syncthreads();
-      }
-    }
+    const bool ok = chunk_sweep<T, R, FWD>(
+        f, F, INV, t.a, nrhs, FWD ? Yf : Z + f.y_off * nrhs, Ls0, Xs0, sm,
+        [&](int row, int r) {
+          return FWD ? __ldcg(Z + g[row] + (int64_t)r * n)
+                     : __ldcg(Yf + row + (int64_t)r * f.p);
+        },
+        [&](int row, int r, T v) {
+          if (!FWD) X[g[row] + (int64_t)r * ldx] = (double)v;
+        },
+        err);
+    if (!ok) break;
     if (!FWD) {
       // this chunk's x is in X: count it for the children's tasks
-      __threadfence();
       __syncthreads();
-      if (tid == 0) atomicAdd(ctr + 2 * nfronts + t.front, 1);
+      if (tid == 0) count_one(ctr + 2 * nfronts + t.front);
     }
   }
   cp_async_wait_all();

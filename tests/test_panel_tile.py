@@ -39,10 +39,12 @@ def test_dense_fronts(gpu, n, precision):
 @pytest.mark.parametrize("n", [7, 40, 64])
 @pytest.mark.parametrize("exponent", [-128, -126, 113, 118])
 def test_fp32_pivots_near_the_exponent_range(gpu, n, exponent):
-    # diagonal near 2n 2^exponent: below 2^-118 or above 2^117
+    # diagonal near 2n 2^exponent: below 2^-118 or above 2^117 (the static
+    # pivot off, which would replace the small ones)
     A, rp, ci, v = _dense(n, 3, 2.0 ** exponent)
-    b = np.random.default_rng(2).uniform(-1, 1, n) * 2.0 ** exponent
-    with snu.Solver(nleaves=2, precision=snu.FP32_IR) as s:
+    # (right-hand sides and solutions stay normal FP32 numbers)
+    b = np.random.default_rng(2).uniform(-1, 1, n) * 2.0 ** max(exponent, 0)
+    with snu.Solver(nleaves=2, precision=snu.FP32_IR, pivot_eps=0.0) as s:
         x = s.construct(rp, ci, v).factorize().solve(b)
         assert s.stats()["fp64_fallback"] == 0
     ref = np.linalg.solve(A, b)
