@@ -408,6 +408,20 @@ class CudaEngine : public Engine {
     }
     if ((rc = upload(d_fr_, frh_))) return rc;
     if ((rc = upload(d_gidx_, fp.gidx))) return rc;
+    {
+      // elimination order of the rows (each is the pivot of one front): the
+      // original row of every position, the position of every front index
+      std::vector<int> orig((size_t)std::max(n_, 1), 0), pos((size_t)std::max(n_, 1), 0);
+      std::vector<int> yidx(fp.gidx.size());
+      for (int f = 0; f < nfronts_; f++)
+        for (int t = 0; t < fp.fronts[f].p; t++) {
+          const int g = fp.gidx[fp.fronts[f].idx_offset + t];
+          orig[frh_[f].y_off + t] = g;
+          pos[g] = (int)(frh_[f].y_off + t);
+        }
+      for (size_t k = 0; k < yidx.size(); k++) yidx[k] = pos[fp.gidx[k]];
+      if ((rc = upload(d_yorig_, orig)) || (rc = upload(d_yidx_, yidx))) return rc;
+    }
     if ((rc = upload(d_rel_, fp.rel))) return rc;
     if ((rc = upload(d_asm_pos_, fp.asm_pos))) return rc;
     if ((rc = upload(d_asm_val_, fp.asm_val))) return rc;
@@ -1022,7 +1036,7 @@ class CudaEngine : public Engine {
   // at most what the device holds at once, blocks stride over the tasks.
   template <typename T, int R>
   int diag_launch(bool fwd, const SweepTask* tasks, int ntasks, const T* F,
-                  const T* I, int nrhs, T* W, T* Y, double* X, int ldx,
+                  const T* I, SweepVec vec, int nrhs, T* W, T* Y, double* X, int ldx,
                   cudaStream_t st) {
     auto k = fwd ? k_fwd_diag<T, R> : k_bwd_diag<T, R>;
     // one task chain per column group of R columns
@@ -1040,8 +1054,8 @@ class CudaEngine : public Engine {
     int* ctr = d_tflags_ + ctr_off_ + 2 * std::max(cur_level_, 0) + (fwd ? 0 : 1);
     ++launches_;
     CK(cudaLaunchKernelEx(&cfg, k, tasks, ntasks, ngroups,
-                          (const FrontDev*)d_fr_, F, I, nrhs, (const T*)W, Y,
-                          (const int*)d_gidx_, X, ldx, ctr, d_flags_ + 4));
+                          (const FrontDev*)d_fr_, F, I, vec, nrhs, (const T*)W,
+                          Y, (const int*)d_gidx_, X, ldx, ctr, d_flags_ + 4));
     return ENG_OK;
   }
   template <typename T, int R>
@@ -1080,12 +1094,13 @@ class CudaEngine : public Engine {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int* ctr = d_sctl_;
-    int* next = ctr + 3 * (int64_t)nfronts_ + (fwd ? 0 : 1);
+    int* next = ctr + 2 * (int64_t)nfronts_ + (fwd ? 0 : 1);
     ++launches_;
     CK(cudaLaunchKernelEx(&cfg, k, (const SolveTask*)(fwd ? d_fwd_tasks_ : d_bwd_tasks_),
                           ntasks, (const FrontDev*)d_fr_, (const SweepDep*)d_dep_,
-                          (const int*)d_gidx_, F, I, nfronts_, nrhs, n_, Z, Y, X,
-                          ldx, ctr, next, d_flags_ + 4));
+                          (const int*)d_gidx_, (const int*)d_yidx_, F, I,
+                          nfronts_, nrhs, (int64_t)n_, Z, Y, X, ldx, ctr, next,
+                          d_flags_ + 4));
     return ENG_OK;
   }
   template <typename T>
@@ -1102,17 +1117,17 @@ class CudaEngine : public Engine {
   // (X: the backward sweep's pivot solutions also go there, ldx apart;
   // null for none)
   int diag_sweep(bool fwd, const SweepTask* tasks, int ntasks, const T* F,
-                 const T* I, int nrhs, T* W, T* Y, double* X, int ldx,
-                 cudaStream_t st) {
+                 const T* I, SweepVec vec, int nrhs, T* W, T* Y, double* X,
+                 int ldx, cudaStream_t st) {
     if (nrhs > SOLVE_COLS) {
       err_ = "pivot-block sweep called with more than 64 right-hand sides";
       return ENG_EINVAL;
     }
-    if (nrhs <= 1) return diag_launch<T, 1>(fwd, tasks, ntasks, F, I, nrhs, W, Y, X, ldx, st);
-    if (nrhs <= 2) return diag_launch<T, 2>(fwd, tasks, ntasks, F, I, nrhs, W, Y, X, ldx, st);
-    if (nrhs <= 4) return diag_launch<T, 4>(fwd, tasks, ntasks, F, I, nrhs, W, Y, X, ldx, st);
-    if (nrhs <= 8) return diag_launch<T, 8>(fwd, tasks, ntasks, F, I, nrhs, W, Y, X, ldx, st);
-    return diag_launch<T, 16>(fwd, tasks, ntasks, F, I, nrhs, W, Y, X, ldx, st);
+    if (nrhs <= 1) return diag_launch<T, 1>(fwd, tasks, ntasks, F, I, vec, nrhs, W, Y, X, ldx, st);
+    if (nrhs <= 2) return diag_launch<T, 2>(fwd, tasks, ntasks, F, I, vec, nrhs, W, Y, X, ldx, st);
+    if (nrhs <= 4) return diag_launch<T, 4>(fwd, tasks, ntasks, F, I, vec, nrhs, W, Y, X, ldx, st);
+    if (nrhs <= 8) return diag_launch<T, 8>(fwd, tasks, ntasks, F, I, vec, nrhs, W, Y, X, ldx, st);
+    return diag_launch<T, 16>(fwd, tasks, ntasks, F, I, vec, nrhs, W, Y, X, ldx, st);
   }
 
   // --------------------------------------------------------- profiling
@@ -1885,7 +1900,7 @@ class CudaEngine : public Engine {
     return ENG_OK;
   }
 
-  // Work vectors of a solve of nrhs columns: W and Y (FP64 for fp64, else
+  // Vectors of a solve of nrhs columns: W (or Z) and Y (FP64 for fp64, else
   // FP32) for one pass of up to pass_cols() columns, the FP64 residual and
   // correction for all columns.  Buffers only grow; a grown
   // buffer replaces (and frees) the smaller one.
@@ -1904,7 +1919,8 @@ class CudaEngine : public Engine {
   int ensure_solve(int nrhs, bool fp64) {
     int rc;
     const size_t g = (size_t)std::min(nrhs, pass_cols());  // one pass
-    const size_t w = (size_t)wtot_ * g, y = (size_t)ytot_ * g;
+    const size_t w = (size_t)(work_vectors() ? wtot_ : ytot_) * g,
+                 y = (size_t)ytot_ * g;
     const size_t r = (size_t)n_ * nrhs;
     if (fp64) {
       if ((rc = grow(d_W64_, wcap64_, w)) || (rc = grow(d_Y64_, ycap64_, y)))
@@ -2172,8 +2188,7 @@ class CudaEngine : public Engine {
   }
 
   // The solve of up to RG columns as two whole-tree sweeps (forward,
-  // backward; see sweep_fused.cuh).  W serves as Z (n x nrhs: the work
-  // vectors hold at least n entries per column).
+  // backward; see sweep_fused.cuh).  W serves as Z.
   template <typename T>
   int tree_solve_fused(const T* F, const T* I, T* W, T* Y, const double* B,
                        int ldb, double* X, int ldx, int nrhs, cudaStream_t st) {
@@ -2187,7 +2202,8 @@ class CudaEngine : public Engine {
     CK(cudaMemsetAsync(d_sctl_, 0, sizeof(int) * sctl_size_, st));
     CK(cudaMemsetAsync(Y, 0xff, sizeof(T) * ytot_ * nrhs, st));  // (SweepNan)
     const int64_t tot = (int64_t)n_ * nrhs;
-    k_sweep_init<T><<<(int)((tot + 255) / 256), 256, 0, st>>>(n_, nrhs, B, ldb, W);
+    k_sweep_init<T><<<(int)((tot + 255) / 256), 256, 0, st>>>(n_, nrhs, d_yorig_, B,
+                                                              ldb, W);
     CKL();
     int rc;
     if ((rc = fused_launch<T>(true, F, I, nrhs, W, Y, nullptr, ldx, st))) return rc;
@@ -2215,7 +2231,6 @@ class CudaEngine : public Engine {
       while (a >= 0 && fp.fronts[a].p == 0) a = fp.fronts[a].parent;
       dep[f].effpar = a;
       dep[f].need = 0;
-      dep[f].nch = (fi.p + DIAG_ROWS - 1) / DIAG_ROWS;
       const bool off = fi.p > 0 && fi.q > 0;
       ngl[f] = off ? ((fi.q + GEMV_ROWS - 1) / GEMV_ROWS) * ((fi.p + GEMV_K - 1) / GEMV_K) : 0;
       dep[f].ngq = off ? ((fi.p + GEMV_ROWS - 1) / GEMV_ROWS) * ((fi.q + GEMV_K - 1) / GEMV_K) : 0;
@@ -2223,6 +2238,7 @@ class CudaEngine : public Engine {
     }
     for (int f = 0; f < nf; f++)
       if (fp.fronts[f].p > 0 && dep[f].effpar >= 0) dep[dep[f].effpar].need += ngl[f];
+    auto chunks = [&](int f) { return (fp.fronts[f].p + DIAG_ROWS - 1) / DIAG_ROWS; };
     std::vector<SolveTask> fw, bw;
     std::vector<std::vector<int>> byp(nlevels_);
     for (int l = 0; l < nlevels_; l++) {
@@ -2234,7 +2250,7 @@ class CudaEngine : public Engine {
     }
     for (int l = 0; l < nlevels_; l++) {
       for (int f : byp[l])
-        for (int c = 0; c < dep[f].nch; c++) fw.push_back({0, f, c, 0});
+        for (int c = 0; c < chunks(f); c++) fw.push_back({0, f, c, 0});
       for (int f : byp[l]) {
         const FrontInfo& fi = fp.fronts[f];
         if (!ngl[f]) continue;
@@ -2252,7 +2268,7 @@ class CudaEngine : public Engine {
             bw.push_back({1, f, a, b});
       }
       for (int f : byp[l])
-        for (int c = dep[f].nch - 1; c >= 0; c--) bw.push_back({0, f, c, 0});
+        for (int c = chunks(f) - 1; c >= 0; c--) bw.push_back({0, f, c, 0});
     }
     nfwd_ = (int)fw.size();
     nbwd_ = (int)bw.size();
@@ -2260,7 +2276,7 @@ class CudaEngine : public Engine {
     if ((rc = upload(d_dep_, dep))) return rc;
     if ((rc = upload(d_fwd_tasks_, fw))) return rc;
     if ((rc = upload(d_bwd_tasks_, bw))) return rc;
-    sctl_size_ = 3 * (int64_t)nf + 2;
+    sctl_size_ = 2 * (int64_t)nf + 2;
     return alloc(d_sctl_, (size_t)sctl_size_);
   }
 
@@ -2274,6 +2290,8 @@ class CudaEngine : public Engine {
     CK(cudaMemsetAsync(d_tflags_, 0, sizeof(int) * tflags_size_, st));
     CK(cudaMemsetAsync(Y, 0xff, sizeof(T) * ytot_ * nrhs, st));  // (SweepNan)
     int rc;
+    if (!work_vectors())
+      return sweep_direct<T>(F, I, W, Y, B, ldb, X, ldx, nrhs, st);
     if ((rc = sweep_levels<T>(lv_, 0, true, true, F, I, W, Y, B, ldb, X, ldx,
                               nrhs, st)))
       return rc;
@@ -2281,8 +2299,67 @@ class CudaEngine : public Engine {
                            nrhs, st);
   }
 
-  // One direction of the level-by-level sweeps over the fronts of a
-  // schedule (forward from the leaves, backward from the root).  ctr_off
+  // Whether solves run on per-front work vectors (a fixed order of the
+  // additions, or an exchange between ranks) rather than on vectors in
+  // elimination order, which need neither extend-adds nor gathers.
+  bool work_vectors() const { return deterministic_ || opt_.dist_world > 1; }
+
+  // Both level-by-level sweeps on vectors in elimination order (W serves as
+  // Z): per level one pivot-block and one off-diagonal launch.
+  template <typename T>
+  int sweep_direct(const T* F, const T* I, T* Z, T* Y, const double* B, int ldb,
+                   double* X, int ldx, int nrhs, cudaStream_t st) {
+    const double es = sizeof(T);
+    const SweepVec vec{n_, d_yidx_};
+    const int64_t tot = (int64_t)n_ * nrhs;
+    int pi, rc;
+    ctr_off_ = 0;
+    cur_level_ = -1;
+    pi = prof_begin(KF_SOLVE_MISC, st);
+    k_sweep_init<T><<<(int)((tot + 255) / 256), 256, 0, st>>>(n_, nrhs, d_yorig_, B,
+                                                              ldb, Z);
+    CKL();
+    prof_end(pi, KF_SOLVE_MISC, st, 0, tot * (es + 8) + 4.0 * n_);
+    for (int dir = 0; dir < 2; dir++) {
+      const bool fwd = dir == 0;
+      if (!fwd) CK(cudaMemsetAsync(Z, 0xff, sizeof(T) * tot, st));  // (SweepNan)
+      for (int k = 0; k < nlevels_; k++) {
+        const int l = fwd ? k : nlevels_ - 1 - k;
+        const LevelSched& L = lv_[l];
+        cur_level_ = l;
+        for (int part = 0; part < 2; part++) {
+          if ((part == 0) == fwd) {  // forward first, backward last
+            if (!(fwd ? L.nwf : L.nwb)) continue;
+            pi = prof_begin(KF_SOLVE_DIAG, st);
+            if ((rc = diag_sweep<T>(fwd, fwd ? L.wf : L.wb, fwd ? L.nwf : L.nwb,
+                                    F, I, vec, nrhs, fwd ? Z : Y, fwd ? Y : Z,
+                                    fwd ? nullptr : X, ldx, st)))
+              return rc;
+            prof_end(pi, KF_SOLVE_DIAG, st, 2.0 * L.diag_elems * nrhs,
+                     L.diag_elems * es);
+            continue;
+          }
+          const int ng = fwd ? L.ngl : L.ngq;
+          if (!ng) continue;
+          pi = prof_begin(KF_SOLVE_GEMM, st);
+          if (fwd)
+            SNU_RG_DISPATCH(nrhs, k_gemv_l21, T, (ng * col_groups(nrhs), 256, 0, st),
+                            (L.gl, col_groups(nrhs), d_fr_, F, vec, nrhs, Z, Y));
+          else
+            SNU_RG_DISPATCH(nrhs, k_gemv_u12, T, (ng * col_groups(nrhs), 256, 0, st),
+                            (L.gq, col_groups(nrhs), d_fr_, F, vec, nrhs, Z, Y));
+          CKL();
+          prof_end(pi, KF_SOLVE_GEMM, st, 2.0 * L.gq_elems * nrhs,
+                   L.gq_elems * es);
+        }
+      }
+    }
+    cur_level_ = -1;
+    return ENG_OK;
+  }
+
+  // One direction of the level-by-level sweeps with per-front work vectors
+  // over the fronts of a schedule (forward from the leaves, backward from the root).  ctr_off
   // selects the schedule's task counters; init: the forward sweep first
   // loads B into each level's fronts (off for fronts whose work vectors
   // were set up and summed across ranks beforehand).
@@ -2292,6 +2369,7 @@ class CudaEngine : public Engine {
                    const double* B, int ldb, double* X, int ldx, int nrhs,
                    cudaStream_t st) {
     const double es = sizeof(T);
+    const SweepVec vec{0, nullptr};
     int pi, rc;
     ctr_off_ = ctr_off;
     if (fwd) {
@@ -2327,7 +2405,7 @@ class CudaEngine : public Engine {
         prof_end(pi, KF_SOLVE_MISC, st, 0, L.solve_elems * nrhs * (es + 12));
         if (L.nwf) {
           pi = prof_begin(KF_SOLVE_DIAG, st);
-          if ((rc = diag_sweep<T>(true, L.wf, L.nwf, F, I, nrhs, W, Y, nullptr,
+          if ((rc = diag_sweep<T>(true, L.wf, L.nwf, F, I, vec, nrhs, W, Y, nullptr,
                                   0, st)))
             return rc;
           prof_end(pi, KF_SOLVE_DIAG, st, 2.0 * L.diag_elems * nrhs,
@@ -2336,7 +2414,7 @@ class CudaEngine : public Engine {
         if (L.ngl) {
           pi = prof_begin(KF_SOLVE_GEMM, st);
           SNU_RG_DISPATCH(nrhs, k_gemv_l21, T, (L.ngl * col_groups(nrhs), 256, 0, st),
-                          (L.gl, col_groups(nrhs), d_fr_, F, nrhs, W, Y));
+                          (L.gl, col_groups(nrhs), d_fr_, F, vec, nrhs, W, Y));
           CKL();
           prof_end(pi, KF_SOLVE_GEMM, st, 2.0 * L.gq_elems * nrhs,
                    L.gq_elems * es);
@@ -2356,7 +2434,7 @@ class CudaEngine : public Engine {
         if (L.ngq) {
           pi = prof_begin(KF_SOLVE_GEMM, st);
           SNU_RG_DISPATCH(nrhs, k_gemv_u12, T, (L.ngq * col_groups(nrhs), 256, 0, st),
-                          (L.gq, col_groups(nrhs), d_fr_, F, nrhs, W, Y));
+                          (L.gq, col_groups(nrhs), d_fr_, F, vec, nrhs, W, Y));
           CKL();
           prof_end(pi, KF_SOLVE_GEMM, st, 2.0 * L.gq_elems * nrhs,
                    L.gq_elems * es);
@@ -2364,7 +2442,7 @@ class CudaEngine : public Engine {
         if (L.nwb) {
           pi = prof_begin(KF_SOLVE_DIAG, st);
           // (the pivot solutions go to X there: the final unpermute)
-          if ((rc = diag_sweep<T>(false, L.wb, L.nwb, F, I, nrhs, W, Y, X, ldx,
+          if ((rc = diag_sweep<T>(false, L.wb, L.nwb, F, I, vec, nrhs, W, Y, X, ldx,
                                   st)))
             return rc;
           prof_end(pi, KF_SOLVE_DIAG, st, 2.0 * L.diag_elems * nrhs,
@@ -2929,6 +3007,8 @@ class CudaEngine : public Engine {
   float* d_Y32_ = nullptr;
   std::vector<FrontDev> frh_;
   FrontDev* d_fr_ = nullptr;
+  // rows in elimination order: original row of each, row of each front index
+  int *d_yorig_ = nullptr, *d_yidx_ = nullptr;
   int *d_gidx_ = nullptr, *d_rel_ = nullptr, *d_asm_val_ = nullptr;
   int64_t* d_asm_pos_ = nullptr;
   int *d_rowptr_ = nullptr, *d_colidx_ = nullptr;

@@ -2,8 +2,19 @@
 // core_trsm / core_update_b / trsm_Lxb / gemm on b in the factorization, and
 // the back solve, SnuMat_factorize.cu:258-345, kernel_sparse.cu:915-944).
 //
-// Per front the work vector W (dim x nrhs) and the pivot part Y (p x nrhs)
-// are updated.  Each level of a sweep is two launches:
+// The vectors of a sweep are n x nrhs, column-major, with the rows in
+// elimination order (a front's pivots are rows [y_off, y_off + p)): Z, the
+// right-hand side that a front's products update in place, in the rows of
+// whichever ancestors pivot them, and Y, the forward result.  The backward
+// sweep updates Y in place and leaves the solution in Z.  yidx maps every
+// front index to its row.
+//
+// Where updates must be added in a fixed order (bit-reproducible runs) or
+// exchanged between ranks, every front has its own work vector W (dim x
+// nrhs) and pivot part of Y (p x nrhs) instead, and the update vectors go
+// from front to front (k_solve_ea).  SweepVec addresses both.
+//
+// Each level of a sweep is two launches (more with work vectors):
 //
 // * the pivot block (rows and columns [0, p)): one cooperative launch over
 //   (front, 128-row chunk) tasks.  The chunk holding a tile's rows solves the
@@ -15,7 +26,7 @@
 //   staged into shared memory with cp.async while it waits.
 // * the off-diagonal part (L21 y for the forward sweep, U12 x_Q for the
 //   backward sweep): a tall-skinny product over (front, 64-row, 256-column)
-//   blocks that adds into W with atomics.
+//   blocks that adds into Z, Y or W with atomics.
 #pragma once
 #include "kernels.cuh"
 
@@ -102,6 +113,28 @@ __device__ __forceinline__ void stage_inv(T* Xs, const T* inv) {
   for (int e = threadIdx.x; e < NB * NB / V; e += blockDim.x)
     cp_async16(Xs + e * V, inv + e * V);
 }
+
+// Where a front's rows are in the vectors of a sweep: n > 0: vectors in
+// elimination order, 0: per-front work vectors and pivot parts.
+struct SweepVec {
+  int n;
+  const int* yidx;  // row of every front index (n > 0)
+  // first pivot row of front f and the distance of its columns
+  __device__ __forceinline__ int64_t piv(const FrontDev& f, int nrhs) const {
+    return n ? f.y_off : f.y_off * nrhs;
+  }
+  __device__ __forceinline__ int64_t ldp(const FrontDev& f) const {
+    return n ? n : f.p;
+  }
+  // the same of its work vector (whose pivot rows start from the right-hand
+  // side: Z with n > 0)
+  __device__ __forceinline__ int64_t work(const FrontDev& f, int nrhs) const {
+    return n ? f.y_off : f.w_off * nrhs;
+  }
+  __device__ __forceinline__ int64_t ldw(const FrontDev& f) const {
+    return n ? n : f.p + f.q;
+  }
+};
 
 // The NaN that marks an element of Y that is not solved yet: every bit set,
 // so a buffer is marked by a memset.  A result with those bits (a NaN that
@@ -200,8 +233,7 @@ __device__ __forceinline__ void lds(const T* p, T (&v)[N]) {
 //   backward, tile s (from the last): x_s = Uinv_s w[k0:k1];
 //            w[r] -= U[r, k0:k1] x_s, r < k0
 // init(row, r): the chunk's starting right-hand side; done(row, r, v): what
-// else becomes of a solved element; Yp (leading dimension f.p, column r0
-// first): where tiles are published and waited for.
+// else becomes of a solved element; Yp (columns ldy apart, column r0 first): where tiles are published and waited for.
 //
 // The chain of tiles is bound by the hand-over between CTAs and by shared
 // memory, which serves 128 requested bytes a cycle, broadcasts included.
@@ -215,8 +247,8 @@ template <typename T, int R, bool FWD, typename Init, typename Done>
 __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
                                             const T* __restrict__ F,
                                             const T* __restrict__ INV,
-                                            int chunk, int nr, T* Yp, T* Ls0,
-                                            T* Xs0, ChunkSmem<T, R>& sm,
+                                            int chunk, int nr, T* Yp,
+                                            int64_t ldy, T* Ls0, T* Xs0, ChunkSmem<T, R>& sm,
                                             Init init, Done done, int* err) {
   constexpr int V = 16 / sizeof(T), RS = ChunkSmem<T, R>::RS;
   constexpr int TC = R >= 4 ? R / 4 : 1, TR = R / TC;  // register tile
@@ -333,7 +365,7 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
             const bool in = i < kb && r < nr;
             ys[i][r] = in ? acc[a][c] : (T)0;
             if (in) {
-              SweepNan<T>::publish(Yp + k0 + i + (int64_t)r * f.p, acc[a][c]);
+              SweepNan<T>::publish(Yp + k0 + i + r * ldy, acc[a][c]);
               done(k0 + i, r, acc[a][c]);
             }
           }
@@ -344,7 +376,7 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
       T v[N];
       auto off = [&](int q) -> int64_t {
         const int e = tid + DIAG_ROWS * q, i = e % NB, r = e / NB;
-        return i < kb && r < nr ? k0 + i + (int64_t)r * f.p : -1;
+        return i < kb && r < nr ? k0 + i + r * ldy : -1;
       };
       if (!poll_all<T, N>(Yp, off, v, err)) sm.bad = 1;
 #pragma unroll
@@ -404,15 +436,16 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
 // descending) order, so every chunk waits only on tasks of lower index; the
 // grid is co-resident (cooperative launch) and blocks take tasks from a
 // counter as they come free, so tasks start in ascending order, which rules
-// out a cycle of waits.  The pivot rows of W are dead after the forward
-// sweep (Y carries the result); the backward sweep also writes the final
-// solution to X in original row order.
+// out a cycle of waits.  A chunk's right-hand side comes from W (forward Z,
+// backward Y, or the work vectors) and its tiles go to Y (forward Y, backward
+// Z, or the pivot parts); the backward sweep also writes the final solution
+// to X in original row order.
 template <typename T, int R, bool FWD>
 __device__ __forceinline__ void diag_sweep_body(
     const SweepTask* __restrict__ tasks, int nbase, int ngroups,
     const FrontDev* __restrict__ fr, const T* __restrict__ F,
-    const T* __restrict__ INV, int nrhs, const T* __restrict__ W, T* Y,
-    const int* __restrict__ gidx, double* __restrict__ X, int ldx,
+    const T* __restrict__ INV, SweepVec vec, int nrhs, const T* __restrict__ W,
+    T* Y, const int* __restrict__ gidx, double* __restrict__ X, int ldx,
     int* next_task, int* err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Ls0 = reinterpret_cast<T*>(smem_raw);  // [2][NB][DIAG_ROWS]
@@ -434,13 +467,13 @@ __device__ __forceinline__ void diag_sweep_body(
     const SweepTask t = tasks[task - g * nbase];
     const int r0 = g * R, nr = min(R, nrhs - r0);
     const FrontDev f = fr[t.front];
-    const T* Wf = W + f.w_off * nrhs + (int64_t)r0 * (f.p + f.q);
-    T* Yf = Y + f.y_off * nrhs + (int64_t)r0 * f.p;
-    const int dim = f.p + f.q;
+    const int64_t ldw = vec.ldw(f), ldy = vec.ldp(f);
+    const T* Wf = W + vec.work(f, nrhs) + r0 * ldw;
+    T* Yf = Y + vec.piv(f, nrhs) + r0 * ldy;
     const int* gi = gidx + f.idx_off;
     const bool ok = chunk_sweep<T, R, FWD>(
-        f, F, INV, t.chunk, nr, Yf, Ls0, Xs0, sm,
-        [&](int row, int r) { return Wf[row + (int64_t)r * dim]; },
+        f, F, INV, t.chunk, nr, Yf, ldy, Ls0, Xs0, sm,
+        [&](int row, int r) { return Wf[row + r * ldw]; },
         [&](int row, int r, T v) {
           if (!FWD && X) X[gi[row] + (int64_t)(r0 + r) * ldx] = (double)v;
         },
@@ -454,22 +487,22 @@ template <typename T, int R>
 __global__ void __launch_bounds__(DIAG_ROWS)
     k_fwd_diag(const SweepTask* __restrict__ tasks, int nbase, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
-               const T* __restrict__ INV, int nrhs, const T* __restrict__ W,
-               T* Y, const int* __restrict__ gidx, double* __restrict__ X,
-               int ldx, int* next_task, int* err) {
-  diag_sweep_body<T, R, true>(tasks, nbase, ngroups, fr, F, INV, nrhs, W, Y,
-                              gidx, X, ldx, next_task, err);
+               const T* __restrict__ INV, SweepVec vec, int nrhs,
+               const T* __restrict__ W, T* Y, const int* __restrict__ gidx,
+               double* __restrict__ X, int ldx, int* next_task, int* err) {
+  diag_sweep_body<T, R, true>(tasks, nbase, ngroups, fr, F, INV, vec, nrhs, W,
+                              Y, gidx, X, ldx, next_task, err);
 }
 
 template <typename T, int R>
 __global__ void __launch_bounds__(DIAG_ROWS)
     k_bwd_diag(const SweepTask* __restrict__ tasks, int nbase, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
-               const T* __restrict__ INV, int nrhs, const T* __restrict__ W,
-               T* Y, const int* __restrict__ gidx, double* __restrict__ X,
-               int ldx, int* next_task, int* err) {
-  diag_sweep_body<T, R, false>(tasks, nbase, ngroups, fr, F, INV, nrhs, W, Y,
-                               gidx, X, ldx, next_task, err);
+               const T* __restrict__ INV, SweepVec vec, int nrhs,
+               const T* __restrict__ W, T* Y, const int* __restrict__ gidx,
+               double* __restrict__ X, int ldx, int* next_task, int* err) {
+  diag_sweep_body<T, R, false>(tasks, nbase, ngroups, fr, F, INV, vec, nrhs, W,
+                               Y, gidx, X, ldx, next_task, err);
 }
 
 // Backward start of a front: W[0:p] = Y (the forward result; Y is marked
@@ -508,8 +541,9 @@ constexpr int GEMV_ROWS = 64, GEMV_K = 256;
 // CTA; the column blocks of a front add into W with atomics.  kchunk -1:
 // the CTA runs over every column block itself, so each row of W has one
 // writer (the bit-reproducible schedule).
-//   FWD:  W[p + i] -= L21[i, :] Y        (i < q, over the p pivot columns)
-//   !FWD: W[i]     -= U12[i, :] W[p:dim] (i < p, over the q update columns)
+//   FWD:  Z[row of p + i] -= L21[i, :] Y    (i < q, over the p pivot columns)
+//   !FWD: Y[i] -= U12[i, :] Z[rows of Q]    (i < p, over the q update columns)
+// With work vectors: W[p + i] -= L21[i, :] Y and W[i] -= U12[i, :] W[p:dim].
 // Blocks of one task are neighbours (they share its factor entries in L2)
 // and take columns [g R, g R + R) of the pass each.
 //
@@ -521,9 +555,9 @@ template <typename T, int R, bool FWD>
 __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
                                          int ngroups,
                                          const FrontDev* __restrict__ fr,
-                                         const T* __restrict__ F, int nrhs,
-                                         T* __restrict__ W,
-                                         const T* __restrict__ Y) {
+                                         const T* __restrict__ F, SweepVec vec,
+                                         int nrhs, T* __restrict__ W,
+                                         T* __restrict__ Y) {
   constexpr int RS = ChunkSmem<T, R>::RS;
   constexpr int KW = GEMV_K / 8;  // columns per warp
   constexpr int UB = R <= 4 ? 16 : 8;  // columns in flight (two rows each)
@@ -537,19 +571,23 @@ __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
   const SweepTask t = tasks[blockIdx.x / ngroups];
   const int r0 = (blockIdx.x % ngroups) * R, nr = min(R, nrhs - r0);
   const FrontDev f = fr[t.front];
-  const int dim = f.p + f.q;
   const int nrows = FWD ? f.q : f.p, nk = FWD ? f.p : f.q;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i0 = t.chunk * GEMV_ROWS + lane;  // rows i0 and i0 + 32
   const int nkb = (nk + GEMV_K - 1) / GEMV_K;
   const int kb0 = t.kchunk < 0 ? 0 : t.kchunk,
             kb1 = t.kchunk < 0 ? nkb : t.kchunk + 1;
-  T* Wf = W + f.w_off * nrhs + (int64_t)r0 * dim;
-  // source vector (ld lds) and the operand block's first element
-  const T* src = FWD ? Y + f.y_off * nrhs + (int64_t)r0 * f.p : Wf + f.p;
-  const int lds_ = FWD ? f.p : dim;
+  // source and destination vectors (columns lsrc / ldst apart; with vec.n
+  // the Q rows, src backward and dst forward, go through yidx), and the
+  // operand block's first element
+  const int64_t lq = vec.ldw(f), lp = FWD ? vec.ldp(f) : lq;
+  T* q0 = W + (vec.n ? 0 : f.w_off * nrhs + f.p) + r0 * lq;
+  T* p0 = FWD || vec.n ? Y + vec.piv(f, nrhs) + r0 * lp : W + f.w_off * nrhs + r0 * lp;
+  const T* src = FWD ? p0 : q0;
+  T* dst = FWD ? q0 : p0;
+  const int64_t lsrc = FWD ? lp : lq, ldst = FWD ? lq : lp;
+  const int* qrow = vec.n ? vec.yidx + f.idx_off + f.p : nullptr;
   const T* a = FWD ? F + f.off + f.p + i0 : F + f.off + i0 + (int64_t)f.p * f.ld;
-  T* dst = FWD ? Wf + f.p : Wf;
   const bool in0 = i0 < nrows, in1 = i0 + 32 < nrows;
   T acc[2][R];
 #pragma unroll
@@ -568,10 +606,13 @@ __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
     };
     load(w0);
     if (kb > kb0) __syncthreads();  // the previous block's slice is read
-#pragma unroll
-    for (int r = 0; r < R; r++) {
+    {
       const int k = threadIdx.x;
-      ys[k][r] = kc0 + k < kc1 && r < nr ? src[kc0 + k + (int64_t)r * lds_] : (T)0;
+      const bool ink = kc0 + k < kc1;
+      const int64_t row = !FWD && qrow && ink ? qrow[kc0 + k] : kc0 + k;
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        ys[k][r] = ink && r < nr ? src[row + r * lsrc] : (T)0;
     }
     __syncthreads();
 #pragma unroll 1
@@ -611,9 +652,10 @@ __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
   __syncthreads();
   for (int e = threadIdx.x; e < GEMV_ROWS * R; e += 256) {
     const int i = e % GEMV_ROWS, r = e / GEMV_ROWS;
-    if (t.chunk * GEMV_ROWS + i < nrows && r < nr) {
+    const int row = t.chunk * GEMV_ROWS + i;
+    if (row < nrows && r < nr) {
       const T s = (red[0][i][r] + red[1][i][r]) + (red[2][i][r] + red[3][i][r]);
-      atomicAdd(dst + t.chunk * GEMV_ROWS + i + (int64_t)r * dim, -s);
+      atomicAdd(dst + (FWD && qrow ? qrow[row] : row) + r * ldst, -s);
     }
   }
 }
@@ -622,16 +664,16 @@ template <typename T, int R>
 __global__ void __launch_bounds__(256)
     k_gemv_l21(const SweepTask* __restrict__ tasks, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
-               int nrhs, T* __restrict__ W, const T* __restrict__ Y) {
-  gemv_off<T, R, true>(tasks, ngroups, fr, F, nrhs, W, Y);
+               SweepVec vec, int nrhs, T* __restrict__ W, T* __restrict__ Y) {
+  gemv_off<T, R, true>(tasks, ngroups, fr, F, vec, nrhs, W, Y);
 }
 
 template <typename T, int R>
 __global__ void __launch_bounds__(256)
     k_gemv_u12(const SweepTask* __restrict__ tasks, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
-               int nrhs, T* __restrict__ W, const T* __restrict__ Y) {
-  gemv_off<T, R, false>(tasks, ngroups, fr, F, nrhs, W, Y);
+               SweepVec vec, int nrhs, T* __restrict__ W, T* __restrict__ Y) {
+  gemv_off<T, R, false>(tasks, ngroups, fr, F, vec, nrhs, W, Y);
 }
 
 }  // namespace snu

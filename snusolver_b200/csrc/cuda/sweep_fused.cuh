@@ -7,23 +7,19 @@
 // latency.  Here every level's work is one task list and a front starts as
 // soon as what it reads is final:
 //
-// * forward: Z (n x nrhs, indexed by original row, precision T) starts as B.
-//   Pivot-block chunk task (f, c): waits until every off-diagonal task of
-//   f's children has finished, gathers its rows of Z, solves the tile chain
-//   of f's pivot block (chunk_sweep: the chunks of f hand tiles over through
-//   Y_f) and writes Y_f.  Off-diagonal task (f, 64-row block, 256-column
-//   block): waits for its columns of Y_f, then
-//   Z[gidx[p + i]] -= L21[i, :] Y_f with atomics -- straight into the rows
-//   of whichever ancestor pivots them (no extend-add: the elimination tree
-//   guarantees only f's descendants update f's pivot rows).
-// * backward: off-diagonal task (f, 64-row block of P, 256-column block of
-//   Q): waits until f's nearest ancestor with pivots has finished its pivot
-//   block (then every ancestor has), reads x_Q from X (FP64) and
-//   Y_f[i] -= U12[i, :] x_Q with atomics.  Pivot-block chunk task: waits for
-//   all of f's off-diagonal tasks, solves the chain with the tile inverses
-//   (descending), writes x_P to X[gidx[...]] (FP64) and hands tiles over
-//   through Z, which the forward sweep is done with (marked unsolved again
-//   between the sweeps).
+// * forward: Z (elimination order, as in sweep.cuh) starts as B.  Pivot-block
+//   chunk task (f, c): waits until every off-diagonal task of f's children
+//   has finished, solves the tile chain of f's pivot block (chunk_sweep: the
+//   chunks of f hand tiles over through Y_f) and writes Y_f.  Off-diagonal
+//   task (f, 64-row block, 256-column block): waits for its columns of Y_f,
+//   then subtracts L21[i, :] Y_f from the rows of Z with atomics -- straight
+//   into the rows of whichever ancestor pivots them (no extend-add: the
+//   elimination tree guarantees only f's descendants update f's pivot rows).
+// * backward: Z is marked unsolved again.  Off-diagonal task (f, 64-row block
+//   of P, 256-column block of Q): waits for its rows of Z (ancestors'
+//   solutions), Y_f[i] -= U12[i, :] Z with atomics.  Pivot-block chunk task:
+//   waits for all of f's off-diagonal tasks, solves the chain with the tile
+//   inverses (descending), writes x_P to Z and, in FP64, to X[gidx[...]].
 //
 // A front's "children" here are its nearest descendants with pivots (fronts
 // without pivots pass their rows on; dep.effpar skips them).  Tasks are
@@ -50,13 +46,11 @@ struct SweepDep {
   int effpar;  // nearest ancestor with pivots (-1: none)
   int need;    // forward: off-diagonal tasks of the fronts whose effpar is f
   int ngq;     // backward: off-diagonal tasks of f
-  int nch;     // pivot-block chunks of f
 };
 
 // Counters of one sweep (zeroed before it), per front: [0, nf) forward
 // off-diagonal tasks finished of f's children, [nf, 2nf) backward
-// off-diagonal tasks of f finished, [2nf, 3nf) backward pivot chunks of f
-// finished.
+// off-diagonal tasks of f finished.
 __device__ __forceinline__ bool wait_count(const int* ctr, int target,
                                            int* err) {
   for (long it = 0; it < WAVE_SPIN_LIMIT; it++) {
@@ -84,13 +78,14 @@ constexpr size_t fused_smem() {
 }
 
 // One off-diagonal block with DIAG_ROWS threads: 64 rows x 2 k-groups.
-// FWD: dst[gidx[p + i]] -= L21[i, kc0:kc1] Y[kc0:kc1]   (Z, ld n)
-// !FWD: Y[i] -= U12[i, kc0:kc1] X[gidx[p + kc0:kc1]]   (X FP64, ld ldx)
+// FWD: Z[rows of p + i] -= L21[i, kc0:kc1] Y[kc0:kc1]
+// !FWD: Y[i] -= U12[i, kc0:kc1] Z[rows of p + kc0:kc1]
+// (q: the rows of Q; Yf: f's rows of Y; columns of both n apart)
 template <typename T, int R, bool FWD>
 __device__ __forceinline__ void fused_offdiag(
-    const FrontDev& f, const T* __restrict__ F, const int* __restrict__ g,
-    int blk, int kblk, int nrhs, T* Z, int n, T* Yf, const double* X,
-    int ldx, unsigned char* sm, int* err) {
+    const FrontDev& f, const T* __restrict__ F, const int* __restrict__ q,
+    int blk, int kblk, int nrhs, T* Z, int64_t n, T* Yf, unsigned char* sm,
+    int* err) {
   constexpr size_t YS = sizeof(T) * GEMV_K * R;
   T(*ys)[R] = reinterpret_cast<T(*)[R]>(sm);
   T(*red)[GEMV_ROWS][R + 1] = reinterpret_cast<T(*)[GEMV_ROWS][R + 1]>(sm + YS);
@@ -101,30 +96,23 @@ __device__ __forceinline__ void fused_offdiag(
   for (int r0 = 0; r0 < nrhs; r0 += R) {
     const int nr = min(R, nrhs - r0);
     __syncthreads();  // the previous pass's reduction is read
-    if (FWD) {  // published by this launch's pivot chunks
-      constexpr int N = GEMV_K * R / DIAG_ROWS, U = N < 8 ? N : 8;
+    // published by this launch's pivot chunks
+    constexpr int N = GEMV_K * R / DIAG_ROWS, U = N < 8 ? N : 8;
 #pragma unroll 1
-      for (int q0 = 0; q0 < N; q0 += U) {
-        T v[U];
-        auto off = [&](int q) -> int64_t {
-          const int e = threadIdx.x + DIAG_ROWS * (q0 + q), k = e % GEMV_K,
-                    r = e / GEMV_K;
-          return kc0 + k < kc1 && r < nr ? kc0 + k + (int64_t)(r0 + r) * f.p : -1;
-        };
-        // (a timeout is in *err; the values are then as good as any)
-        poll_all<T, U>(Yf, off, v, err);
+    for (int q0 = 0; q0 < N; q0 += U) {
+      T v[U];
+      auto off = [&](int u) -> int64_t {
+        const int e = threadIdx.x + DIAG_ROWS * (q0 + u), k = kc0 + e % GEMV_K,
+                  r = e / GEMV_K;
+        if (k >= kc1 || r >= nr) return -1;
+        return (FWD ? k : q[k]) + (r0 + r) * n;
+      };
+      // (a timeout is in *err; the values are then as good as any)
+      poll_all<T, U>(FWD ? Yf : Z, off, v, err);
 #pragma unroll
-        for (int q = 0; q < U; q++) {
-          const int e = threadIdx.x + DIAG_ROWS * (q0 + q);
-          ys[e % GEMV_K][e / GEMV_K] = off(q) >= 0 ? v[q] : (T)0;
-        }
-      }
-    } else {
-      for (int e = threadIdx.x; e < GEMV_K * R; e += blockDim.x) {
-        const int k = e % GEMV_K, r = e / GEMV_K;
-        ys[k][r] = kc0 + k < kc1 && r < nr
-                       ? (T)__ldcg(X + g[f.p + kc0 + k] + (int64_t)(r0 + r) * ldx)
-                       : (T)0;
+      for (int u = 0; u < U; u++) {
+        const int e = threadIdx.x + DIAG_ROWS * (q0 + u);
+        ys[e % GEMV_K][e / GEMV_K] = off(u) >= 0 ? v[u] : (T)0;
       }
     }
     __syncthreads();
@@ -155,9 +143,9 @@ __device__ __forceinline__ void fused_offdiag(
       for (int r = 0; r < nr; r++) {
         const T s = red[0][threadIdx.x][r] + red[1][threadIdx.x][r];
         if (FWD)
-          atomicAdd(Z + g[f.p + i] + (int64_t)(r0 + r) * n, -s);
+          atomicAdd(Z + q[i] + (r0 + r) * n, -s);
         else
-          atomicAdd(Yf + i + (int64_t)(r0 + r) * f.p, -s);
+          atomicAdd(Yf + i + (r0 + r) * n, -s);
       }
     }
   }
@@ -168,10 +156,10 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     k_sweep_fused(const SolveTask* __restrict__ tasks, int ntasks,
                   const FrontDev* __restrict__ fr,
                   const SweepDep* __restrict__ dep,
-                  const int* __restrict__ gidx, const T* __restrict__ F,
-                  const T* __restrict__ INV, int nfronts, int nrhs, int n,
-                  T* Z, T* Y, double* X, int ldx, int* ctr, int* next_task,
-                  int* err) {
+                  const int* __restrict__ gidx, const int* __restrict__ yidx,
+                  const T* __restrict__ F, const T* __restrict__ INV,
+                  int nfronts, int nrhs, int64_t n, T* Z, T* Y, double* X,
+                  int ldx, int* ctr, int* next_task, int* err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Ls0 = reinterpret_cast<T*>(smem_raw);  // [2][NB][DIAG_ROWS]
   T* Xs0 = Ls0 + 2 * NB * DIAG_ROWS;         // [2][NB * NB]
@@ -190,18 +178,11 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     const FrontDev f = fr[t.front];
     const SweepDep d = dep[t.front];
     const int* g = gidx + f.idx_off;
-    T* Yf = Y + f.y_off * nrhs;
+    T* Yf = Y + f.y_off;
     if (t.kind == 1) {
       // ------------------------------------------ off-diagonal block
-      if (!FWD) {  // the ancestors' x is final
-        if (tid == 0 && d.effpar >= 0 &&
-            !wait_count(ctr + 2 * nfronts + d.effpar, dep[d.effpar].nch, err))
-          sm.bad = 1;
-        __syncthreads();
-        if (sm.bad) return;
-      }
-      fused_offdiag<T, R, FWD>(f, F, g, t.a, t.b, nrhs, Z, n, Yf, X, ldx,
-                               smem_raw, err);
+      fused_offdiag<T, R, FWD>(f, F, yidx + f.idx_off + f.p, t.a, t.b, nrhs, Z,
+                               n, Yf, smem_raw, err);
       __syncthreads();
       if (tid == 0) {  // (the release orders the CTA's atomics before it)
         if (!FWD)
@@ -219,36 +200,31 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     }
     __syncthreads();
     if (sm.bad) return;
-    // the chunk's rows: forward from Z (gathered), backward from Y_f (the
-    // forward result less U12 x_Q); both written by this launch: via L2
+    // the chunk's rows: forward from Z, backward from Y (the forward result
+    // less U12 x_Q); both written by this launch: via L2
+    T* Zf = Z + f.y_off;
     const bool ok = chunk_sweep<T, R, FWD>(
-        f, F, INV, t.a, nrhs, FWD ? Yf : Z + f.y_off * nrhs, Ls0, Xs0, sm,
-        [&](int row, int r) {
-          return FWD ? __ldcg(Z + g[row] + (int64_t)r * n)
-                     : __ldcg(Yf + row + (int64_t)r * f.p);
-        },
+        f, F, INV, t.a, nrhs, FWD ? Yf : Zf, n, Ls0, Xs0, sm,
+        [&](int row, int r) { return __ldcg((FWD ? Zf : Yf) + row + r * n); },
         [&](int row, int r, T v) {
           if (!FWD) X[g[row] + (int64_t)r * ldx] = (double)v;
         },
         err);
     if (!ok) break;
-    if (!FWD) {
-      // this chunk's x is in X: count it for the children's tasks
-      __syncthreads();
-      if (tid == 0) count_one(ctr + 2 * nfronts + t.front);
-    }
   }
   cp_async_wait_all();
 }
 
-// Z = (T) B: the forward sweep's starting vector.
+// Z = (T) B in elimination order (orig: the original row of every row): the
+// forward sweep's starting vector.
 template <typename T>
-__global__ void k_sweep_init(int n, int nrhs, const double* __restrict__ B,
-                             int ldb, T* __restrict__ Z) {
+__global__ void k_sweep_init(int n, int nrhs, const int* __restrict__ orig,
+                             const double* __restrict__ B, int ldb,
+                             T* __restrict__ Z) {
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= (int64_t)n * nrhs) return;
   const int i = (int)(e % n), r = (int)(e / n);
-  Z[e] = (T)B[i + (int64_t)r * ldb];
+  Z[e] = (T)B[orig[i] + (int64_t)r * ldb];
 }
 
 }  // namespace snu
