@@ -191,18 +191,6 @@ constexpr int GBM = 64, GBN = 64;
 // outer block of the two-level blocked partial LU (a multiple of NB)
 constexpr int OB = OB_COLS;
 
-#define SNU_LAUNCH_(K, T, R, CFG, ARGS) K<T, R><<<SNU_UNPACK CFG>>> ARGS
-#define SNU_UNPACK(...) __VA_ARGS__
-// Launch a sweep kernel specialized for the right-hand-side group width.
-#define SNU_RG_DISPATCH(nrhs, K, T, CFG, ARGS)        \
-  do {                                                \
-    if ((nrhs) <= 1) SNU_LAUNCH_(K, T, 1, CFG, ARGS);  \
-    else if ((nrhs) <= 2) SNU_LAUNCH_(K, T, 2, CFG, ARGS); \
-    else if ((nrhs) <= 4) SNU_LAUNCH_(K, T, 4, CFG, ARGS); \
-    else if ((nrhs) <= 8) SNU_LAUNCH_(K, T, 8, CFG, ARGS); \
-    else SNU_LAUNCH_(K, T, 16, CFG, ARGS);             \
-  } while (0)
-
 class CudaEngine : public Engine {
  public:
   explicit CudaEngine(const EngineOptions& o) : opt_(o) {}
@@ -1032,8 +1020,48 @@ class CudaEngine : public Engine {
     return ENG_OK;
   }
 
-  // One cooperative launch of the pivot-block sweep of a level: the grid is
-  // at most what the device holds at once, blocks stride over the tasks.
+  // Launch of a sweep kernel that may start while the kernel before it in the
+  // stream still runs (see grid_wait): its launch latency and the first loads
+  // of factors, which no kernel of a solve writes, overlap that kernel's end.
+  static cudaLaunchConfig_t chained_config(int grid, int block, size_t smem,
+                                           cudaStream_t st,
+                                           cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+  }
+  // One off-diagonal product launch of a level.
+  template <typename T, int R>
+  int gemv_launch_r(bool fwd, const SweepTask* tasks, int ntasks, const T* F,
+                    SweepVec vec, int nrhs, T* W, T* Y, cudaStream_t st) {
+    auto k = fwd ? k_gemv_l21<T, R> : k_gemv_u12<T, R>;
+    const int ngroups = (nrhs + R - 1) / R;
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = chained_config(ntasks * ngroups, 256, 0, st, at);
+    ++launches_;
+    CK(cudaLaunchKernelEx(&cfg, k, tasks, ngroups, (const FrontDev*)d_fr_, F, vec,
+                          nrhs, W, Y));
+    return ENG_OK;
+  }
+  template <typename T>
+  int gemv_launch(bool fwd, const SweepTask* tasks, int ntasks, const T* F,
+                  SweepVec vec, int nrhs, T* W, T* Y, cudaStream_t st) {
+    if (nrhs <= 1) return gemv_launch_r<T, 1>(fwd, tasks, ntasks, F, vec, nrhs, W, Y, st);
+    if (nrhs <= 2) return gemv_launch_r<T, 2>(fwd, tasks, ntasks, F, vec, nrhs, W, Y, st);
+    if (nrhs <= 4) return gemv_launch_r<T, 4>(fwd, tasks, ntasks, F, vec, nrhs, W, Y, st);
+    if (nrhs <= 8) return gemv_launch_r<T, 8>(fwd, tasks, ntasks, F, vec, nrhs, W, Y, st);
+    return gemv_launch_r<T, 16>(fwd, tasks, ntasks, F, vec, nrhs, W, Y, st);
+  }
+
+  // One launch of the pivot-block sweep of a level: the grid is at most what
+  // the device holds at once, blocks take tasks from a counter.
   template <typename T, int R>
   int diag_launch(bool fwd, const SweepTask* tasks, int ntasks, const T* F,
                   const T* I, SweepVec vec, int nrhs, T* W, T* Y, double* X, int ldx,
@@ -1041,16 +1069,10 @@ class CudaEngine : public Engine {
     auto k = fwd ? k_fwd_diag<T, R> : k_bwd_diag<T, R>;
     // one task chain per column group of R columns
     const int ngroups = (nrhs + R - 1) / R;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(std::min(ntasks * ngroups, coop_cap_[(const void*)k]));
-    cfg.blockDim = dim3(DIAG_ROWS);
-    cfg.dynamicSmemBytes = sweep_smem<T>();
-    cfg.stream = st;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cudaLaunchConfig_t cfg = chained_config(
+        std::min(ntasks * ngroups, coop_cap_[(const void*)k]), DIAG_ROWS,
+        sweep_smem<T>(), st, at);
     int* ctr = d_tflags_ + ctr_off_ + 2 * std::max(cur_level_, 0) + (fwd ? 0 : 1);
     ++launches_;
     CK(cudaLaunchKernelEx(&cfg, k, tasks, ntasks, ngroups,
@@ -2133,9 +2155,6 @@ class CudaEngine : public Engine {
   // Columns per solve pass: SOLVE_COLS for the level-by-level sweeps, RG
   // for the whole-tree sweeps (they hold a chunk's rows for RG columns).
   int pass_cols() const { return fused_solve_ ? RG : SOLVE_COLS; }
-  // Register groups of a pass of nrhs columns (the sweep kernels' R is
-  // nrhs rounded up to a power of two up to RG, then RG).
-  static int col_groups(int nrhs) { return nrhs <= RG ? 1 : (nrhs + RG - 1) / RG; }
 
   // tree_solve over passes of at most `group` columns (0: pass_cols());
   // W and Y, sized for one pass, are reused by every pass.
@@ -2342,13 +2361,8 @@ class CudaEngine : public Engine {
           const int ng = fwd ? L.ngl : L.ngq;
           if (!ng) continue;
           pi = prof_begin(KF_SOLVE_GEMM, st);
-          if (fwd)
-            SNU_RG_DISPATCH(nrhs, k_gemv_l21, T, (ng * col_groups(nrhs), 256, 0, st),
-                            (L.gl, col_groups(nrhs), d_fr_, F, vec, nrhs, Z, Y));
-          else
-            SNU_RG_DISPATCH(nrhs, k_gemv_u12, T, (ng * col_groups(nrhs), 256, 0, st),
-                            (L.gq, col_groups(nrhs), d_fr_, F, vec, nrhs, Z, Y));
-          CKL();
+          if ((rc = gemv_launch<T>(fwd, fwd ? L.gl : L.gq, ng, F, vec, nrhs, Z, Y, st)))
+            return rc;
           prof_end(pi, KF_SOLVE_GEMM, st, 2.0 * L.gq_elems * nrhs,
                    L.gq_elems * es);
         }
@@ -2413,9 +2427,8 @@ class CudaEngine : public Engine {
         }
         if (L.ngl) {
           pi = prof_begin(KF_SOLVE_GEMM, st);
-          SNU_RG_DISPATCH(nrhs, k_gemv_l21, T, (L.ngl * col_groups(nrhs), 256, 0, st),
-                          (L.gl, col_groups(nrhs), d_fr_, F, vec, nrhs, W, Y));
-          CKL();
+          if ((rc = gemv_launch<T>(true, L.gl, L.ngl, F, vec, nrhs, W, Y, st)))
+            return rc;
           prof_end(pi, KF_SOLVE_GEMM, st, 2.0 * L.gq_elems * nrhs,
                    L.gq_elems * es);
         }
@@ -2433,9 +2446,8 @@ class CudaEngine : public Engine {
         prof_end(pi, KF_SOLVE_MISC, st, 0, L.solve_elems * nrhs * (es + 12));
         if (L.ngq) {
           pi = prof_begin(KF_SOLVE_GEMM, st);
-          SNU_RG_DISPATCH(nrhs, k_gemv_u12, T, (L.ngq * col_groups(nrhs), 256, 0, st),
-                          (L.gq, col_groups(nrhs), d_fr_, F, vec, nrhs, W, Y));
-          CKL();
+          if ((rc = gemv_launch<T>(false, L.gq, L.ngq, F, vec, nrhs, W, Y, st)))
+            return rc;
           prof_end(pi, KF_SOLVE_GEMM, st, 2.0 * L.gq_elems * nrhs,
                    L.gq_elems * es);
         }

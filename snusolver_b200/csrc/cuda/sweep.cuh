@@ -114,6 +114,19 @@ __device__ __forceinline__ void stage_inv(T* Xs, const T* inv) {
     cp_async16(Xs + e * V, inv + e * V);
 }
 
+// Programmatic dependent launch: a sweep kernel may start while the one
+// before it in the stream still runs.  Until grid_wait it touches only what no
+// kernel of a solve writes (task lists, fronts, factors) and its own task
+// counter, zeroed before the first kernel of the pass.  The vectors are no
+// __restrict__ pointers: loads from one that a kernel only reads could be
+// moved before the wait.
+__device__ __forceinline__ void grid_start_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Where a front's rows are in the vectors of a sweep: n > 0: vectors in
 // elimination order, 0: per-front work vectors and pivot parts.
 struct SweepVec {
@@ -243,7 +256,7 @@ __device__ __forceinline__ void lds(const T* p, T (&v)[N]) {
 // through its values alone: no fence, flag or second load.  With the
 // products below, 64 columns on a 54^3 grid 20.1 -> 15.6 ms (pivot blocks
 // 9.5 -> 6.5, products 5.8 -> 3.9), 13 FP64 columns on 37^3 2.44 -> 1.66 ms.
-template <typename T, int R, bool FWD, typename Init, typename Done>
+template <typename T, int R, bool FWD, bool WAIT, typename Init, typename Done>
 __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
                                             const T* __restrict__ F,
                                             const T* __restrict__ INV,
@@ -284,6 +297,7 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
   cp_async_commit();
   if (sA != sB) stage(sA + ds);
   cp_async_commit();
+  if (WAIT) grid_wait();  // (nothing the previous kernel writes so far)
   T w[NP][VW][TC];
 #pragma unroll
   for (int p = 0; p < NP; p++)
@@ -434,9 +448,9 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
 // Forward (FWD) or backward sweep of the pivot blocks of one level.  Tasks
 // are (front, chunk) with the chunks of a front in ascending (backward:
 // descending) order, so every chunk waits only on tasks of lower index; the
-// grid is co-resident (cooperative launch) and blocks take tasks from a
-// counter as they come free, so tasks start in ascending order, which rules
-// out a cycle of waits.  A chunk's right-hand side comes from W (forward Z,
+// blocks take tasks from a counter as they come free, so tasks start in
+// ascending order and the lowest unfinished one never waits on a task that is
+// not running, whatever part of the grid is resident.  A chunk's right-hand side comes from W (forward Z,
 // backward Y, or the work vectors) and its tiles go to Y (forward Y, backward
 // Z, or the pivot parts); the backward sweep also writes the final solution
 // to X in original row order.
@@ -444,8 +458,8 @@ template <typename T, int R, bool FWD>
 __device__ __forceinline__ void diag_sweep_body(
     const SweepTask* __restrict__ tasks, int nbase, int ngroups,
     const FrontDev* __restrict__ fr, const T* __restrict__ F,
-    const T* __restrict__ INV, SweepVec vec, int nrhs, const T* __restrict__ W,
-    T* Y, const int* __restrict__ gidx, double* __restrict__ X, int ldx,
+    const T* __restrict__ INV, SweepVec vec, int nrhs, const T* W,
+    T* Y, const int* __restrict__ gidx, double* X, int ldx,
     int* next_task, int* err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Ls0 = reinterpret_cast<T*>(smem_raw);  // [2][NB][DIAG_ROWS]
@@ -453,6 +467,7 @@ __device__ __forceinline__ void diag_sweep_body(
   __shared__ ChunkSmem<T, R> sm;
   __shared__ int s_task;
   if (threadIdx.x == 0) sm.bad = 0;
+  grid_start_next();
   for (;;) {
     // tasks start in ascending order as blocks come free
     cp_async_wait_all();
@@ -471,9 +486,9 @@ __device__ __forceinline__ void diag_sweep_body(
     const T* Wf = W + vec.work(f, nrhs) + r0 * ldw;
     T* Yf = Y + vec.piv(f, nrhs) + r0 * ldy;
     const int* gi = gidx + f.idx_off;
-    const bool ok = chunk_sweep<T, R, FWD>(
+    const bool ok = chunk_sweep<T, R, FWD, true>(
         f, F, INV, t.chunk, nr, Yf, ldy, Ls0, Xs0, sm,
-        [&](int row, int r) { return Wf[row + r * ldw]; },
+        [&](int row, int r) { return __ldcg(Wf + row + r * ldw); },
         [&](int row, int r, T v) {
           if (!FWD && X) X[gi[row] + (int64_t)(r0 + r) * ldx] = (double)v;
         },
@@ -481,6 +496,8 @@ __device__ __forceinline__ void diag_sweep_body(
     if (!ok) break;
   }
   cp_async_wait_all();
+  grid_wait();  // (also by a block without a task: the kernel's end is then
+                // behind the end of the one before it)
 }
 
 template <typename T, int R>
@@ -488,8 +505,8 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     k_fwd_diag(const SweepTask* __restrict__ tasks, int nbase, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
                const T* __restrict__ INV, SweepVec vec, int nrhs,
-               const T* __restrict__ W, T* Y, const int* __restrict__ gidx,
-               double* __restrict__ X, int ldx, int* next_task, int* err) {
+               const T* W, T* Y, const int* __restrict__ gidx,
+               double* X, int ldx, int* next_task, int* err) {
   diag_sweep_body<T, R, true>(tasks, nbase, ngroups, fr, F, INV, vec, nrhs, W,
                               Y, gidx, X, ldx, next_task, err);
 }
@@ -499,8 +516,8 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     k_bwd_diag(const SweepTask* __restrict__ tasks, int nbase, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
                const T* __restrict__ INV, SweepVec vec, int nrhs,
-               const T* __restrict__ W, T* Y, const int* __restrict__ gidx,
-               double* __restrict__ X, int ldx, int* next_task, int* err) {
+               const T* W, T* Y, const int* __restrict__ gidx,
+               double* X, int ldx, int* next_task, int* err) {
   diag_sweep_body<T, R, false>(tasks, nbase, ngroups, fr, F, INV, vec, nrhs, W,
                                Y, gidx, X, ldx, next_task, err);
 }
@@ -556,8 +573,8 @@ __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
                                          int ngroups,
                                          const FrontDev* __restrict__ fr,
                                          const T* __restrict__ F, SweepVec vec,
-                                         int nrhs, T* __restrict__ W,
-                                         T* __restrict__ Y) {
+                                         int nrhs, T* W, T* Y) {
+  grid_start_next();
   constexpr int RS = ChunkSmem<T, R>::RS;
   constexpr int KW = GEMV_K / 8;  // columns per warp
   constexpr int UB = R <= 4 ? 16 : 8;  // columns in flight (two rows each)
@@ -605,14 +622,17 @@ __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
       }
     };
     load(w0);
-    if (kb > kb0) __syncthreads();  // the previous block's slice is read
+    if (kb > kb0)
+      __syncthreads();  // the previous block's slice is read
+    else
+      grid_wait();
     {
       const int k = threadIdx.x;
       const bool ink = kc0 + k < kc1;
       const int64_t row = !FWD && qrow && ink ? qrow[kc0 + k] : kc0 + k;
 #pragma unroll
       for (int r = 0; r < R; r++)
-        ys[k][r] = ink && r < nr ? src[row + r * lsrc] : (T)0;
+        ys[k][r] = ink && r < nr ? __ldcg(src + row + r * lsrc) : (T)0;
     }
     __syncthreads();
 #pragma unroll 1
@@ -664,7 +684,7 @@ template <typename T, int R>
 __global__ void __launch_bounds__(256)
     k_gemv_l21(const SweepTask* __restrict__ tasks, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
-               SweepVec vec, int nrhs, T* __restrict__ W, T* __restrict__ Y) {
+               SweepVec vec, int nrhs, T* W, T* Y) {
   gemv_off<T, R, true>(tasks, ngroups, fr, F, vec, nrhs, W, Y);
 }
 
@@ -672,7 +692,7 @@ template <typename T, int R>
 __global__ void __launch_bounds__(256)
     k_gemv_u12(const SweepTask* __restrict__ tasks, int ngroups,
                const FrontDev* __restrict__ fr, const T* __restrict__ F,
-               SweepVec vec, int nrhs, T* __restrict__ W, T* __restrict__ Y) {
+               SweepVec vec, int nrhs, T* W, T* Y) {
   gemv_off<T, R, false>(tasks, ngroups, fr, F, vec, nrhs, W, Y);
 }
 

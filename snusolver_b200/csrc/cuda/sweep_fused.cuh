@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     // the chunk's rows: forward from Z, backward from Y (the forward result
     // less U12 x_Q); both written by this launch: via L2
     T* Zf = Z + f.y_off;
-    const bool ok = chunk_sweep<T, R, FWD>(
+    const bool ok = chunk_sweep<T, R, FWD, false>(
         f, F, INV, t.a, nrhs, FWD ? Yf : Zf, n, Ls0, Xs0, sm,
         [&](int row, int r) { return __ldcg((FWD ? Zf : Yf) + row + r * n); },
         [&](int row, int r, T v) {
