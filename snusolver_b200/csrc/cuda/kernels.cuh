@@ -363,6 +363,30 @@ __global__ void k_residual(int n, const int* __restrict__ rowptr,
   }
 }
 
+// out[seg of row i] = max_i sum_j |A(i, j)|, every row summed in order (the
+// infinity norm of each matrix of a batch; seg null: one matrix).  A NaN row
+// sum counts as 0, like std::max against a running maximum.
+__global__ void k_row_norms(int n, const int* __restrict__ rowptr,
+                            const double* __restrict__ vals,
+                            const int* __restrict__ seg,
+                            unsigned long long* out) {
+  const unsigned full = 0xffffffffu;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double m = 0;
+  if (i < n)
+    for (int k = rowptr[i]; k < rowptr[i + 1]; k++) m += fabs(vals[k]);
+  if (!(m > 0)) m = 0;
+  const int sg = i < n ? (seg ? seg[i] : 0) : -1;
+  const int s0 = __shfl_sync(full, sg, 0);
+  if (__all_sync(full, sg == s0 || sg < 0)) {
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(full, m, o));
+    if ((threadIdx.x & 31) == 0 && s0 >= 0)
+      atomicMax(out + s0, (unsigned long long)__double_as_longlong(m));
+  } else if (sg >= 0) {
+    atomicMax(out + sg, (unsigned long long)__double_as_longlong(m));
+  }
+}
+
 // out[r] = max_i |M(i, r)| (non-negative doubles compare like their bit
 // patterns, so a 64-bit integer atomicMax reduces them).
 __global__ void k_colmax(int n, int nrhs, const double* __restrict__ M, int ld,

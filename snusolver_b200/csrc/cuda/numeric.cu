@@ -4,8 +4,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
-#include <thread>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -414,7 +412,6 @@ class CudaEngine : public Engine {
     if ((rc = upload(d_asm_pos_, fp.asm_pos))) return rc;
     if ((rc = upload(d_asm_val_, fp.asm_val))) return rc;
     std::vector<int> rp(rowptr, rowptr + n_ + 1), ci(colidx, colidx + nnz_);
-    rowptr_h_ = rp;
     if ((rc = upload(d_rowptr_, rp))) return rc;
     if ((rc = upload(d_colidx_, ci))) return rc;
     if ((rc = alloc(d_vals_, (size_t)std::max(1, nnz_)))) return rc;
@@ -444,7 +441,6 @@ class CudaEngine : public Engine {
       err_ = "bad segment boundaries";
       return ENG_EINVAL;
     }
-    seg_start_ = row_start;
     nseg_ = ns;
     if (ns > 1) {
       std::vector<int> seg(n_);
@@ -462,48 +458,21 @@ class CudaEngine : public Engine {
     CK(cudaSetDevice(opt_.device));
     CK(cudaMemcpyAsync(d_vals_, vals, sizeof(double) * nnz_,
                        cudaMemcpyHostToDevice, stream_));
-    // ||A||_inf for the backward error (per matrix of a batch), on host
-    // threads while the copy runs: row chunks of one matrix, or whole
-    // matrices of a batch (each row summed in order: the same norm as a
-    // serial loop)
+    // ||A||_inf for the backward error, per matrix of a batch
+    unsigned long long* d = nseg_ > 1 ? d_segnorms_ : d_norms_;
+    std::vector<unsigned long long> h(nseg_);
+    CK(cudaMemsetAsync(d, 0, sizeof(unsigned long long) * nseg_, stream_));
+    k_row_norms<<<(n_ + 255) / 256, 256, 0, stream_>>>(
+        n_, d_rowptr_, d_vals_, nseg_ > 1 ? d_seg_ : nullptr, d);
+    CKL();
+    CK(cudaMemcpyAsync(h.data(), d, sizeof(unsigned long long) * nseg_,
+                       cudaMemcpyDeviceToHost, stream_));
+    CK(cudaStreamSynchronize(stream_));
     anorm_ = 0;
-    if ((int)anorm_seg_.size() != nseg_) anorm_seg_.assign(nseg_, 0.0);
-    auto rows_max = [&](int i0, int i1) {
-      double a = 0;
-      for (int i = i0; i < i1; i++) {
-        double s = 0;
-        for (int k = rowptr_h_[i]; k < rowptr_h_[i + 1]; k++) s += std::fabs(vals[k]);
-        a = std::max(a, s);
-      }
-      return a;
-    };
-    const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-    const int nt = nnz_ > (1 << 17) ? std::min(hw, 16) : 1;
-    if (nseg_ > 1) {
-      std::atomic<int> next{0};
-      auto work = [&] {
-        for (int b; (b = next.fetch_add(1)) < nseg_;)
-          anorm_seg_[b] = rows_max(seg_start_[b], seg_start_[b + 1]);
-      };
-      std::vector<std::thread> th;
-      for (int t = 1; t < nt; t++) th.emplace_back(work);
-      work();
-      for (auto& x : th) x.join();
-    } else {
-      std::vector<double> part(nt, 0.0);
-      std::vector<std::thread> th;
-      for (int t = 1; t < nt; t++)
-        th.emplace_back([&, t] {
-          part[t] = rows_max((int)((int64_t)n_ * t / nt),
-                             (int)((int64_t)n_ * (t + 1) / nt));
-        });
-      part[0] = rows_max(0, (int)((int64_t)n_ / nt));
-      for (auto& x : th) x.join();
-      anorm_seg_[0] = *std::max_element(part.begin(), part.end());
-    }
+    anorm_seg_.assign(nseg_, 0.0);
+    for (int b = 0; b < nseg_; b++) memcpy(&anorm_seg_[b], &h[b], sizeof(double));
     for (int b = 0; b < nseg_; b++) anorm_ = std::max(anorm_, anorm_seg_[b]);
     have64_ = have32_ = mixed64_ = false;
-    CK(cudaStreamSynchronize(stream_));
     return ENG_OK;
   }
 
@@ -3070,12 +3039,10 @@ class CudaEngine : public Engine {
   std::vector<std::pair<void**, size_t>> fix_;
   // matrices of a batch (segments of rows) and their ||A||inf
   int nseg_ = 1;
-  std::vector<int> seg_start_;
   std::vector<double> anorm_seg_{0.0};
   int* d_seg_ = nullptr;
   unsigned long long* d_segnorms_ = nullptr;
   std::vector<double> bnorm_;
-  std::vector<int> rowptr_h_;
   std::vector<LevelSched> lv_;
 };
 
