@@ -178,11 +178,14 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 }
 
 // FP64 C -= A B (mode 0) or C = A B (mode 1) on the FP64 tensor cores
-// (mma.sync m8n8k4 .f64): the same 64 x 64 tiles and problems as k_gemm, four
-// warps of 32 x 32 each (4 x 4 MMA tiles of 8 x 8), k in steps of 16 staged
-// through shared memory with the next step's loads in flight in registers.
-// A warp reads one A and one B value per lane for every 4 x 4 block of
-// MMAs (16 fused multiply-adds per load, four times the SIMT kernel's).
+// (mma.sync m8n8k4 .f64): the same problems as k_gemm in BT x BT tiles, four
+// warps of BT/2 x BT/2 each, k in steps of 16 staged through shared memory
+// with the next step's loads in flight in registers.  At BT = 64 a warp reads
+// one A and one B value per lane for every 4 x 4 block of MMAs (16 fused
+// multiply-adds per load, four times the SIMT kernel's).  One 64 x 64 x 256
+// tile keeps an SM's FP64 units busy for 8.6 us, so a batch of fewer tiles
+// than fill the device runs in 32 x 32 tiles (the eight Schur launches of a
+// 128^2 grid 230 -> 113 us).
 // Fragment layouts (PTX ISA, mma.m8n8k4 .f64): lane l holds A(l / 4, l % 4),
 // B(l % 4, l / 4) and C(l / 4, 2 (l % 4) + {0, 1}).
 __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
@@ -193,13 +196,14 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
       : "d"(a), "d"(b));
 }
 
+template <int BT>
 __global__ void __launch_bounds__(128)
     k_gemm_dmma(const GemmTile* __restrict__ tiles,
                 const GemmProb* __restrict__ probs,
                 const double* __restrict__ Abase,
                 const double* __restrict__ Bbase, double* __restrict__ Cbase,
                 int mode, const int* __restrict__ rel_base) {
-  constexpr int BM = 64, BN = 64, BK = 16, PAD = 4;
+  constexpr int BM = BT, BN = BT, BK = 16, PAD = 4, MT = BT / 16;
   __shared__ double As[BK][BM + PAD];  // As[k][m]
   __shared__ double Bs[BK][BN + PAD];  // Bs[k][n]
   const GemmTile tl = tiles[blockIdx.x];
@@ -209,13 +213,13 @@ __global__ void __launch_bounds__(128)
   const double* B = Bbase + P.b;
   double* C = Cbase + P.c;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;  // warp tile origin
+  const int wm = (warp & 1) * (BT / 2), wn = (warp >> 1) * (BT / 2);  // warp tile
   const int gr = lane >> 2, gc = lane & 3;                // fragment coords
-  double acc[4][4][2];
+  double acc[MT][MT][2];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < MT; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < MT; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
   // loads: A tile BM x BK (8 per thread, rows contiguous), B tile BK x BN
   // (8 per thread, k contiguous)
   constexpr int LA = BM * BK / 128, LB = BK * BN / 128;
@@ -250,25 +254,25 @@ __global__ void __launch_bounds__(128)
     if (k0 + BK < P.k) gload(k0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 4) {
-      double a[4], b[4];
+      double a[MT], b[MT];
 #pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[kk + gc][wm + 8 * i + gr];
+      for (int i = 0; i < MT; i++) a[i] = As[kk + gc][wm + 8 * i + gr];
 #pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[kk + gc][wn + 8 * j + gr];
+      for (int j = 0; j < MT; j++) b[j] = Bs[kk + gc][wn + 8 * j + gr];
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < MT; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) dmma_8x8x4(acc[i][j], a[i], b[j]);
+        for (int j = 0; j < MT; j++) dmma_8x8x4(acc[i][j], a[i], b[j]);
     }
     __syncthreads();
   }
   const int* rel = rel_base + P.rel;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < MT; i++) {
     const int gi = m0 + wm + 8 * i + gr;
     if (gi >= P.m) continue;
 #pragma unroll
-    for (int j = 0; j < 4; j++)
+    for (int j = 0; j < MT; j++)
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int gj = n0 + wn + 8 * j + 2 * gc + h;

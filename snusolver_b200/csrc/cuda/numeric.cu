@@ -86,6 +86,10 @@ struct GemmBatch {
   GemmProb* probs = nullptr;  // all problems (FP64 path, SIMT)
   GemmTile* tiles = nullptr;
   int ntiles = 0;
+  // FP64: the same problems in 32 x 32 tiles, for a batch whose 64 x 64 tiles
+  // do not fill the device
+  GemmTile* tiles32 = nullptr;
+  int ntiles32 = 0;
   double flops = 0;  // sum of 2 m n k
   double elems = 0;  // algorithmic elements moved: A + B read, C read+write
   // FP32 path: problems large enough for the tensor cores, and the rest
@@ -186,6 +190,9 @@ struct LevelSched {
 
 
 constexpr int GBM = 64, GBN = 64;
+// 64 x 64 tiles from which an FP64 batch fills the device (148 SMs, three
+// blocks on each): fewer run as 32 x 32 tiles
+constexpr int DMMA_FILL = 444;
 // outer block of the two-level blocked partial LU (a multiple of NB)
 constexpr int OB = OB_COLS;
 
@@ -1265,9 +1272,9 @@ class CudaEngine : public Engine {
 
   // ---------------------------------------------------------- schedule
   static void tiles_of(const std::vector<GemmProb>& probs,
-                       std::vector<GemmTile>& tiles) {
+                       std::vector<GemmTile>& tiles, int bt = GBM) {
     for (size_t k = 0; k < probs.size(); k++) {
-      int tm = (probs[k].m + GBM - 1) / GBM, tn = (probs[k].n + GBN - 1) / GBN;
+      int tm = (probs[k].m + bt - 1) / bt, tn = (probs[k].n + bt - 1) / bt;
       for (int b = 0; b < tn; b++)
         for (int a = 0; a < tm; a++) tiles.push_back({(int)k, a, b});
     }
@@ -1292,6 +1299,12 @@ class CudaEngine : public Engine {
     int rc;
     if ((rc = upload(gb.probs, probs))) return rc;
     if ((rc = upload(gb.tiles, tiles))) return rc;
+    if (gb.ntiles < DMMA_FILL) {
+      std::vector<GemmTile> t32;
+      tiles_of(probs, t32, 32);
+      gb.ntiles32 = (int)t32.size();
+      if ((rc = upload(gb.tiles32, t32))) return rc;
+    }
     if (fp64_only_build_) return ENG_OK;  // (FP64 schedules: tiles only)
     // FP32 split
     std::vector<GemmProb> rest;
@@ -1940,11 +1953,16 @@ class CudaEngine : public Engine {
                   cudaStream_t st, int fam) {
     if (gb.ntiles == 0) return ENG_OK;
     int pi = prof_begin(fam, st);
-    if (sizeof(T) == 8 && use_dmma_)  // FP64 on the FP64 tensor cores
-      k_gemm_dmma<<<gb.ntiles, 128, 0, st>>>(gb.tiles, gb.probs,
-                                             (const double*)A, (const double*)B,
-                                             (double*)C, mode, d_rel_);
-    else
+    if (sizeof(T) == 8 && use_dmma_) {  // FP64 on the FP64 tensor cores
+      if (gb.ntiles32)
+        k_gemm_dmma<32><<<gb.ntiles32, 128, 0, st>>>(
+            gb.tiles32, gb.probs, (const double*)A, (const double*)B, (double*)C,
+            mode, d_rel_);
+      else
+        k_gemm_dmma<64><<<gb.ntiles, 128, 0, st>>>(
+            gb.tiles, gb.probs, (const double*)A, (const double*)B, (double*)C,
+            mode, d_rel_);
+    } else
       k_gemm<T, GBM, GBN, 16, 4, 4><<<gb.ntiles, 256, 0, st>>>(
           gb.tiles, gb.probs, A, B, C, mode, d_rel_);
     CKL();

@@ -360,7 +360,9 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
           for (int a = 0; a < AR; a++)
             acc[a][0] = (part[0][a] + part[1][a]) + (part[2][a] + part[3][a]);
         } else {
-#pragma unroll 4
+          // (sixteen steps' operands in flight: 64 columns on 54^3 12.4 ms
+          // with four, 12.1 with sixteen)
+#pragma unroll 16
           for (int m = 0; m < NB; m++) {
             T xv[AR], v[C];
             lds(Xs + i0 + m * NB, xv);
@@ -416,7 +418,7 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
         for (int a = 0; a < VW; a++)
 #pragma unroll
           for (int c = 0; c < TC; c++) acc[p][a][c] = (T)0;
-#pragma unroll 4
+#pragma unroll 16
       for (int m = 0; m < kb; m++) {
         T y[TC];
         lds(&ys[m][tc], y);
