@@ -128,7 +128,7 @@ class ClockSampler:
 # capture and its command are summarised in the named file
 PROFILED_TRAFFIC = {
     ("c2_convdiff64", "panel_block"): {
-        "bytes_per_launch": 53.74e6,
+        "bytes_per_launch": 53.80e6,
         "source": "profiles/k_panel_block_dram_c2_convdiff64.md"},
 }
 
