@@ -414,9 +414,12 @@ SNU_API void snu_free(void* p);
 /* ---- self-test (no reference counterpart) ---- */
 /* Every device-side wait of this library (inter-block flags, mbarriers) is
    bounded: after its iteration limit it records an error, the kernel
-   returns and the call reports SNU_ETIMEOUT.  This runs one such wait on a
-   flag that nothing sets and returns its status: SNU_ETIMEOUT (after well
-   under a second) is the expected answer; the device stays usable. */
+   returns and the call reports SNU_ETIMEOUT.  This runs such a wait on a
+   flag that nothing sets, and every wait of the whole-tree sweep on values
+   and counters that nothing publishes, and checks that their blocks hand
+   nothing on and take no other task: SNU_ETIMEOUT is the expected answer,
+   SNU_OK means that a wait did not end so (snu_last_error says which).  The
+   device stays usable. */
 SNU_API snu_status snu_selftest_wait_timeout(int device);
 /* The FP32 tile factorization forms each pivot's reciprocal as a hardware
    approximation refined by one Newton-Raphson step.  This compares it with

@@ -1098,7 +1098,7 @@ class CudaEngine : public Engine {
                           ntasks, (const FrontDev*)d_fr_, (const SweepDep*)d_dep_,
                           (const int*)d_gidx_, (const int*)d_yidx_, F, I,
                           nfronts_, nrhs, (int64_t)n_, Z, Y, X, ldx, ctr, next,
-                          d_flags_ + 4));
+                          d_flags_ + 4, WAVE_SPIN_LIMIT));
     return ENG_OK;
   }
   template <typename T>
@@ -3073,6 +3073,103 @@ __global__ void k_wait_selftest(const int* flag, int* err) {
   if (threadIdx.x == 0) wait_flag(flag, err);
 }
 
+namespace {
+
+// The waits of the whole-tree sweep, made to run out: one front (192 pivots,
+// 64 rows below) whose vectors stay marked unsolved, and a list of two equal
+// tasks for one block.  The wait must give up, the block must record the
+// error, hand nothing on (counters, vectors) and leave the second task.
+// preset: the error is recorded beforehand, so the block has to leave long
+// before its iteration limit, here the full one.  Sets `why` if it did not
+// end so.
+template <typename T, int R, bool FWD>
+cudaError_t sweep_wait_case(SolveTask task, int need, bool preset,
+                            std::string& why) {
+  constexpr int P = 192, Q = 64, N = P + Q;
+  FrontDev f = {};
+  f.p = P;
+  f.q = Q;
+  f.ld = N;
+  f.parent = -1;
+  const SweepDep dep{0, need, need};
+  const SolveTask tasks[2] = {task, task};
+  std::vector<int> idx(N);
+  for (int i = 0; i < N; i++) idx[i] = i;
+  // one allocation: factors and inverses (zero), Z and Y (marked), tables
+  const size_t nf = sizeof(T) * (N * N + 3 * 2 * NB * NB), nv = sizeof(T) * N * R;
+  const size_t oz = nf, oy = oz + nv, oi = oy + nv, of = oi + sizeof(int) * N,
+               ot = of + sizeof(FrontDev), od = ot + sizeof tasks,
+               oc = od + sizeof dep, end = oc + 4 * sizeof(int);
+  static_assert(sizeof(FrontDev) % 8 == 0 && sizeof(SolveTask) % 8 == 0, "");
+  unsigned char* d = nullptr;
+  cudaError_t e = cudaMalloc((void**)&d, end);
+  if (e != cudaSuccess) return e;
+  int ctl[4] = {0, 0, 0, preset ? 1 : 0};  // two counters, next task, error
+  std::vector<unsigned char> v(2 * nv);
+  cudaEvent_t ev[2] = {};
+  float ms = 0;
+  auto k = k_sweep_fused<T, R, FWD>;
+  auto ok = [&](cudaError_t r) { return (e = r) == cudaSuccess; };
+  if (ok(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)fused_smem<T>())) &&
+      ok(cudaMemset(d, 0, nf)) && ok(cudaMemset(d + oz, 0xff, 2 * nv)) &&
+      ok(cudaMemcpy(d + oi, idx.data(), sizeof(int) * N, cudaMemcpyHostToDevice)) &&
+      ok(cudaMemcpy(d + of, &f, sizeof f, cudaMemcpyHostToDevice)) &&
+      ok(cudaMemcpy(d + ot, tasks, sizeof tasks, cudaMemcpyHostToDevice)) &&
+      ok(cudaMemcpy(d + od, &dep, sizeof dep, cudaMemcpyHostToDevice)) &&
+      ok(cudaMemcpy(d + oc, ctl, sizeof ctl, cudaMemcpyHostToDevice)) &&
+      ok(cudaEventCreate(&ev[0])) && ok(cudaEventCreate(&ev[1])) &&
+      ok(cudaEventRecord(ev[0]))) {
+    int* c = (int*)(d + oc);
+    const int* ix = (const int*)(d + oi);
+    const T* F = (const T*)d;
+    k<<<1, DIAG_ROWS, fused_smem<T>()>>>(
+        (const SolveTask*)(d + ot), 2, (const FrontDev*)(d + of),
+        (const SweepDep*)(d + od), ix, ix, F, F + N * N, 1, R, (int64_t)N,
+        (T*)(d + oz), (T*)(d + oy), (double*)nullptr, N, c, c + 2, c + 3,
+        preset ? WAVE_SPIN_LIMIT : 4096L);
+    if (ok(cudaGetLastError()) && ok(cudaEventRecord(ev[1])) &&
+        ok(cudaDeviceSynchronize()) && ok(cudaEventElapsedTime(&ms, ev[0], ev[1])) &&
+        ok(cudaMemcpy(ctl, c, sizeof ctl, cudaMemcpyDeviceToHost)))
+      ok(cudaMemcpy(v.data(), d + oz, 2 * nv, cudaMemcpyDeviceToHost));
+  }
+  for (cudaEvent_t x : ev)
+    if (x) cudaEventDestroy(x);
+  cudaFree(d);
+  if (e != cudaSuccess) return e;
+  const bool kept = std::all_of(v.begin(), v.end(), [](unsigned char b) { return b == 0xff; });
+  if (!ctl[3] || ctl[0] || ctl[1] || ctl[2] != 1 || !kept || ms > 250.f)
+    why = std::string(FWD ? "forward" : "backward") + " sweep, task kind " +
+          std::to_string(task.kind) + ": error " + std::to_string(ctl[3]) +
+          ", counters " + std::to_string(ctl[0]) + " " + std::to_string(ctl[1]) +
+          ", tasks taken " + std::to_string(ctl[2]) + ", vectors " +
+          (kept ? "kept" : "changed") + ", " + std::to_string(ms) + " ms";
+  return cudaSuccess;
+}
+
+// Every wait of the sweep: an off-diagonal block for its source values, the
+// pivot-block chunk of another tile's rows for that tile, and a chunk for its
+// front's counter.
+template <typename T, int R, bool FWD>
+cudaError_t sweep_wait_cases(std::string& why) {
+  const struct {
+    SolveTask task;
+    int need;
+    bool preset;
+  } cases[] = {{{1, 0, 0, 0}, 0, false},
+               {{0, 0, FWD ? 1 : 0, 0}, 0, false},
+               {{0, 0, 0, 0}, 1, false},
+               {{1, 0, 0, 0}, 0, true},
+               {{0, 0, 0, 0}, 1, true}};
+  for (const auto& c : cases) {
+    cudaError_t e = sweep_wait_case<T, R, FWD>(c.task, c.need, c.preset, why);
+    if (e != cudaSuccess || !why.empty()) return e;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace
+
 int wait_selftest(int device, std::string& err) {
   if (cudaSetDevice(device) != cudaSuccess) {
     cudaGetLastError();
@@ -3091,14 +3188,21 @@ int wait_selftest(int device, std::string& err) {
   cudaError_t e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof h, cudaMemcpyDeviceToHost);
   cudaFree(d);
+  std::string why;
+  if (e == cudaSuccess) e = sweep_wait_cases<float, 1, true>(why);
+  if (e == cudaSuccess && why.empty()) e = sweep_wait_cases<float, 16, true>(why);
+  if (e == cudaSuccess && why.empty()) e = sweep_wait_cases<float, 16, false>(why);
+  if (e == cudaSuccess && why.empty()) e = sweep_wait_cases<double, 16, true>(why);
+  if (e == cudaSuccess && why.empty()) e = sweep_wait_cases<double, 16, false>(why);
   if (e != cudaSuccess) {
     err = cudaGetErrorString(e);
     return ENG_ECUDA;
   }
-  if (h[1]) {
-    err = "wait on an unset flag gave up after its iteration limit";
+  if (h[1] && why.empty()) {
+    err = "every wait gave up after its iteration limit";
     return ENG_ETIMEOUT;
   }
+  err = why.empty() ? "the wait on an unset flag did not give up" : why;
   return ENG_OK;
 }
 

@@ -183,14 +183,27 @@ struct SweepNan<double> {
   }
 };
 
+// Whether another wait of the solve has already run out (read through L2; a
+// spinning thread looks every WAVE_ERR_EVERY iterations, so that a launch in
+// which one wait runs out ends soon after it and not a limit per waiting task
+// later).
+constexpr long WAVE_ERR_EVERY = 256;
+__device__ __forceinline__ bool wait_failed(const int* err, long it) {
+  if (it % WAVE_ERR_EVERY != WAVE_ERR_EVERY - 1) return false;
+  int e;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(e) : "l"(err) : "memory");
+  return e != 0;
+}
+
 // v[q] = src[off(q)] for the q that are wanted, once published (bounded
-// spin; all loads in flight together); on timeout sets *err and returns
-// false.
+// spin of `limit` iterations; all loads in flight together); on timeout, or
+// once *err is set, sets *err and returns false: the caller's block leaves
+// its kernel without handing anything on.
 template <typename T, int N, typename Off>
 __device__ __forceinline__ bool poll_all(const T* src, Off off, T (&v)[N],
-                                         int* err) {
+                                         int* err, long limit = WAVE_SPIN_LIMIT) {
   bool again = true;
-  for (long it = 0; again && it < WAVE_SPIN_LIMIT; it++) {
+  for (long it = 0; again && it < limit; it++) {
     again = false;
 #pragma unroll
     for (int q = 0; q < N; q++) {
@@ -199,6 +212,7 @@ __device__ __forceinline__ bool poll_all(const T* src, Off off, T (&v)[N],
     }
 #pragma unroll
     for (int q = 0; q < N; q++) again |= off(q) >= 0 && SweepNan<T>::is(v[q]);
+    if (again && wait_failed(err, it)) break;
     if (again && it > 4) __nanosleep(20);
   }
   if (again) atomicExch(err, 1);
@@ -262,7 +276,8 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
                                             const T* __restrict__ INV,
                                             int chunk, int nr, T* Yp,
                                             int64_t ldy, T* Ls0, T* Xs0, ChunkSmem<T, R>& sm,
-                                            Init init, Done done, int* err) {
+                                            Init init, Done done, int* err,
+                                            long limit = WAVE_SPIN_LIMIT) {
   constexpr int V = 16 / sizeof(T), RS = ChunkSmem<T, R>::RS;
   constexpr int TC = R >= 4 ? R / 4 : 1, TR = R / TC;  // register tile
   constexpr int NG = R / TC, NT = DIAG_ROWS / NG;      // column groups, lanes
@@ -394,7 +409,7 @@ __device__ __forceinline__ bool chunk_sweep(const FrontDev& f,
         const int e = tid + DIAG_ROWS * q, i = e % NB, r = e / NB;
         return i < kb && r < nr ? k0 + i + r * ldy : -1;
       };
-      if (!poll_all<T, N>(Yp, off, v, err)) sm.bad = 1;
+      if (!poll_all<T, N>(Yp, off, v, err, limit)) sm.bad = 1;
 #pragma unroll
       for (int q = 0; q < N; q++) {
         const int e = tid + DIAG_ROWS * q, i = e % NB, r = e / NB;

@@ -28,8 +28,9 @@
 // pivot chunks in descending order), so every wait is on a task of lower
 // index; the grid is co-resident (cooperative launch) and blocks take tasks
 // from a counter in ascending order, so the lowest unfinished task never
-// waits on an unfinished one.  Every wait is bounded (error flag, then the
-// block returns).
+// waits on an unfinished one.  Every wait is bounded: when it runs out, or
+// another block's has, the block records the error and returns, handing on
+// nothing of the task it was in and taking no other.
 #pragma once
 #include "sweep.cuh"
 
@@ -52,12 +53,13 @@ struct SweepDep {
 // off-diagonal tasks finished of f's children, [nf, 2nf) backward
 // off-diagonal tasks of f finished.
 __device__ __forceinline__ bool wait_count(const int* ctr, int target,
-                                           int* err) {
-  for (long it = 0; it < WAVE_SPIN_LIMIT; it++) {
+                                           int* err, long limit) {
+  for (long it = 0; it < limit; it++) {
     int v;
     asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(ctr)
                  : "memory");
     if (v >= target) return true;
+    if (wait_failed(err, it)) break;
     if (it > 4) __nanosleep(20);
   }
   atomicExch(err, 1);
@@ -81,11 +83,13 @@ constexpr size_t fused_smem() {
 // FWD: Z[rows of p + i] -= L21[i, kc0:kc1] Y[kc0:kc1]
 // !FWD: Y[i] -= U12[i, kc0:kc1] Z[rows of p + kc0:kc1]
 // (q: the rows of Q; Yf: f's rows of Y; columns of both n apart)
+// False (in every thread) if a wait ran out: nothing was added then.  bad: the
+// block's shared flag for it, zero before.
 template <typename T, int R, bool FWD>
-__device__ __forceinline__ void fused_offdiag(
+__device__ __forceinline__ bool fused_offdiag(
     const FrontDev& f, const T* __restrict__ F, const int* __restrict__ q,
     int blk, int kblk, int nrhs, T* Z, int64_t n, T* Yf, unsigned char* sm,
-    int* err) {
+    int* bad, int* err, long limit) {
   constexpr size_t YS = sizeof(T) * GEMV_K * R;
   T(*ys)[R] = reinterpret_cast<T(*)[R]>(sm);
   T(*red)[GEMV_ROWS][R + 1] = reinterpret_cast<T(*)[GEMV_ROWS][R + 1]>(sm + YS);
@@ -107,8 +111,10 @@ __device__ __forceinline__ void fused_offdiag(
         if (k >= kc1 || r >= nr) return -1;
         return (FWD ? k : q[k]) + (r0 + r) * n;
       };
-      // (a timeout is in *err; the values are then as good as any)
-      poll_all<T, U>(FWD ? Yf : Z, off, v, err);
+      if (!poll_all<T, U>(FWD ? Yf : Z, off, v, err, limit)) {
+        *bad = 1;
+        break;
+      }
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const int e = threadIdx.x + DIAG_ROWS * (q0 + u);
@@ -116,6 +122,7 @@ __device__ __forceinline__ void fused_offdiag(
       }
     }
     __syncthreads();
+    if (*bad) return false;
     T acc[R];
 #pragma unroll
     for (int r = 0; r < R; r++) acc[r] = (T)0;
@@ -149,6 +156,7 @@ __device__ __forceinline__ void fused_offdiag(
       }
     }
   }
+  return true;
 }
 
 template <typename T, int R, bool FWD>
@@ -159,7 +167,7 @@ __global__ void __launch_bounds__(DIAG_ROWS)
                   const int* __restrict__ gidx, const int* __restrict__ yidx,
                   const T* __restrict__ F, const T* __restrict__ INV,
                   int nfronts, int nrhs, int64_t n, T* Z, T* Y, double* X,
-                  int ldx, int* ctr, int* next_task, int* err) {
+                  int ldx, int* ctr, int* next_task, int* err, long limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Ls0 = reinterpret_cast<T*>(smem_raw);  // [2][NB][DIAG_ROWS]
   T* Xs0 = Ls0 + 2 * NB * DIAG_ROWS;         // [2][NB * NB]
@@ -181,8 +189,10 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     T* Yf = Y + f.y_off;
     if (t.kind == 1) {
       // ------------------------------------------ off-diagonal block
-      fused_offdiag<T, R, FWD>(f, F, yidx + f.idx_off + f.p, t.a, t.b, nrhs, Z,
-                               n, Yf, smem_raw, err);
+      if (!fused_offdiag<T, R, FWD>(f, F, yidx + f.idx_off + f.p, t.a, t.b,
+                                    nrhs, Z, n, Yf, smem_raw, &sm.bad, err,
+                                    limit))
+        break;
       __syncthreads();
       if (tid == 0) {  // (the release orders the CTA's atomics before it)
         if (!FWD)
@@ -194,8 +204,8 @@ __global__ void __launch_bounds__(DIAG_ROWS)
     }
     // ------------------------------------------------ pivot-block chunk
     if (tid == 0) {
-      const bool ok = FWD ? wait_count(ctr + t.front, d.need, err)
-                          : wait_count(ctr + nfronts + t.front, d.ngq, err);
+      const bool ok = FWD ? wait_count(ctr + t.front, d.need, err, limit)
+                          : wait_count(ctr + nfronts + t.front, d.ngq, err, limit);
       if (!ok) sm.bad = 1;
     }
     __syncthreads();
@@ -209,7 +219,7 @@ __global__ void __launch_bounds__(DIAG_ROWS)
         [&](int row, int r, T v) {
           if (!FWD) X[g[row] + (int64_t)r * ldx] = (double)v;
         },
-        err);
+        err, limit);
     if (!ok) break;
   }
   cp_async_wait_all();

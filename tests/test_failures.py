@@ -2,8 +2,10 @@
 
 Host-made failures only (a singular matrix, a memory budget that is too
 small, calls out of order) plus the library's own bounded-wait self-test,
-which waits on a flag nothing sets and must report SNU_ETIMEOUT with the
-device still usable afterwards.  Nothing here traps, faults or hangs a GPU.
+which waits on a flag, counters and values that nothing publishes and must
+report SNU_ETIMEOUT (every wait gave up, and the whole-tree sweep's blocks
+handed nothing on and took no further task) with the device still usable
+afterwards.  Nothing here traps, faults or hangs a GPU.
 """
 import numpy as np
 import pytest
@@ -17,7 +19,8 @@ def test_bounded_wait_reports_timeout_and_device_stays_usable(gpu):
     lib = snu.load_library()
     lib.snu_selftest_wait_timeout.restype = int
     st = lib.snu_selftest_wait_timeout(0)
-    assert st == 4, snu.STATUS.get(st)  # SNU_ETIMEOUT
+    # SNU_ETIMEOUT
+    assert st == 4, (snu.STATUS.get(st), lib.snu_last_error(None))
     # the context is intact: a normal solve still works
     rp, ci, v = generators.laplace2d_perturbed(20, 20, seed=1)
     b = np.ones(400)
