@@ -421,6 +421,11 @@ class CudaEngine : public Engine {
     std::vector<int> rp(rowptr, rowptr + n_ + 1), ci(colidx, colidx + nnz_);
     if ((rc = upload(d_rowptr_, rp))) return rc;
     if ((rc = upload(d_colidx_, ci))) return rc;
+    std::vector<int> longr;  // rows whose norm a block sums
+    for (int i = 0; i < n_; i++)
+      if (rp[i + 1] - rp[i] > ROW_LONG) longr.push_back(i);
+    nlong_ = (int)longr.size();
+    if (nlong_ && (rc = upload(d_long_, longr))) return rc;
     if ((rc = alloc(d_vals_, (size_t)std::max(1, nnz_)))) return rc;
     if ((rc = alloc(d_flags_, 8))) return rc;
     if ((rc = alloc(d_norms_, 3 * 64))) return rc;
@@ -472,6 +477,11 @@ class CudaEngine : public Engine {
     k_row_norms<<<(n_ + 255) / 256, 256, 0, stream_>>>(
         n_, d_rowptr_, d_vals_, nseg_ > 1 ? d_seg_ : nullptr, d);
     CKL();
+    if (nlong_) {
+      k_row_norms_long<<<nlong_, 256, 0, stream_>>>(
+          d_long_, d_rowptr_, d_vals_, nseg_ > 1 ? d_seg_ : nullptr, d);
+      CKL();
+    }
     CK(cudaMemcpyAsync(h.data(), d, sizeof(unsigned long long) * nseg_,
                        cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
@@ -3011,6 +3021,8 @@ class CudaEngine : public Engine {
   int *d_gidx_ = nullptr, *d_rel_ = nullptr, *d_asm_val_ = nullptr;
   int64_t* d_asm_pos_ = nullptr;
   int *d_rowptr_ = nullptr, *d_colidx_ = nullptr;
+  int* d_long_ = nullptr;  // rows of more than ROW_LONG entries
+  int nlong_ = 0;
   double* d_vals_ = nullptr;
   int* d_flags_ = nullptr;
   unsigned long long* d_norms_ = nullptr;
