@@ -86,8 +86,8 @@ struct GemmBatch {
   GemmProb* probs = nullptr;  // all problems (FP64 path, SIMT)
   GemmTile* tiles = nullptr;
   int ntiles = 0;
-  // FP64: the same problems in 32 x 32 tiles, for a batch whose 64 x 64 tiles
-  // do not fill the device
+  // FP64: the same problems in 32 x 32 tiles, for a batch that the device
+  // holds at once in them (see gemm_batch)
   GemmTile* tiles32 = nullptr;
   int ntiles32 = 0;
   double flops = 0;  // sum of 2 m n k
@@ -190,9 +190,6 @@ struct LevelSched {
 
 
 constexpr int GBM = 64, GBN = 64;
-// 64 x 64 tiles from which an FP64 batch fills the device (148 SMs, three
-// blocks on each): fewer run as 32 x 32 tiles
-constexpr int DMMA_FILL = 444;
 // outer block of the two-level blocked partial LU (a multiple of NB)
 constexpr int OB = OB_COLS;
 
@@ -240,6 +237,8 @@ class CudaEngine : public Engine {
                                                        TCP_THREADS,
                                                        tc_smem_bytes<64>()));
       tcp_cap_[1] = std::max(1, std::min(nb, 4)) * sms;  // TMEM: 4 x 128 columns
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gemm_dmma<32>, 128, 0));
+      dmma32_cap_ = (int64_t)nb * sms;
     }
     {
       const char* e = getenv("SNU_TC_GEMM");
@@ -1309,7 +1308,17 @@ class CudaEngine : public Engine {
     int rc;
     if ((rc = upload(gb.probs, probs))) return rc;
     if ((rc = upload(gb.tiles, tiles))) return rc;
-    if (gb.ntiles < DMMA_FILL) {
+    // FP64 batches run in 32 x 32 tiles while the device holds all of those
+    // at once (1480 on 148 SMs): 64 x 64 tiles then leave SMs idle or cover
+    // more padding.  Measured with k = 64, 128 and 256, the Schur scatter and
+    // square problems of 64 to 448 rows, 64 x 64 time / 32 x 32 time: up to
+    // 600 tiles of 32 1.4-2.0, up to 1480 1.04-1.9; from there to 1770, where
+    // a second wave begins while 64 x 64 tiles may still take one, 0.76-1.4;
+    // above that 0.94-1.7 as the 64 x 64 tiles' own waves fall.
+    int64_t n32 = 0;
+    for (const GemmProb& g : probs)
+      n32 += (int64_t)((g.m + 31) / 32) * ((g.n + 31) / 32);
+    if (n32 <= dmma32_cap_) {
       std::vector<GemmTile> t32;
       tiles_of(probs, t32, 32);
       gb.ntiles32 = (int)t32.size();
@@ -2997,6 +3006,7 @@ class CudaEngine : public Engine {
   int force_tcp_ = -1;  // tensor-core kernel variant forced (-1: per batch)
   int force_width_ = -1;  // tensor-core tile width forced (0: 128, 1: 64)
   bool use_dmma_ = true;  // FP64 GEMMs on the FP64 tensor cores
+  int64_t dmma32_cap_ = 0;  // 32 x 32 tiles the device holds at once
   int force_split_ = -1;  // FP32 GEMM split for every batch: 0 TF32x3, 1 BF16x3
   bool deterministic_ = false;  // fixed-order reductions (SNU_DETERMINISTIC)
   int tcp_cap_[2] = {148, 148};  // persistent grid per tile width
