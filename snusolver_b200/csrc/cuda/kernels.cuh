@@ -183,9 +183,9 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 // with the next step's loads in flight in registers.  At BT = 64 a warp reads
 // one A and one B value per lane for every 4 x 4 block of MMAs (16 fused
 // multiply-adds per load, four times the SIMT kernel's).  One 64 x 64 x 256
-// tile keeps an SM's FP64 units busy for 8.6 us, so a batch that the device
-// holds at once in 32 x 32 tiles runs in those (the eight Schur launches of a
-// 128^2 grid 230 -> 113 us).
+// tile keeps an SM's FP64 units busy for 8.6 us, so a batch of few 32 x 32
+// tiles runs in those (the eight Schur launches of a 128^2 grid 230 -> 113
+// us).
 // Fragment layouts (PTX ISA, mma.m8n8k4 .f64): lane l holds A(l / 4, l % 4),
 // B(l % 4, l / 4) and C(l / 4, 2 (l % 4) + {0, 1}).
 __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {

@@ -86,8 +86,8 @@ struct GemmBatch {
   GemmProb* probs = nullptr;  // all problems (FP64 path, SIMT)
   GemmTile* tiles = nullptr;
   int ntiles = 0;
-  // FP64: the same problems in 32 x 32 tiles, for a batch that the device
-  // holds at once in them (see gemm_batch)
+  // FP64: the same problems in 32 x 32 tiles, for a batch of few enough of
+  // them (see gemm_batch)
   GemmTile* tiles32 = nullptr;
   int ntiles32 = 0;
   double flops = 0;  // sum of 2 m n k
@@ -238,7 +238,7 @@ class CudaEngine : public Engine {
                                                        tc_smem_bytes<64>()));
       tcp_cap_[1] = std::max(1, std::min(nb, 4)) * sms;  // TMEM: 4 x 128 columns
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gemm_dmma<32>, 128, 0));
-      dmma32_cap_ = (int64_t)nb * sms;
+      dmma32_cap_ = 2 * (int64_t)nb * sms;  // two rounds of five blocks an SM
     }
     {
       const char* e = getenv("SNU_TC_GEMM");
@@ -1308,13 +1308,15 @@ class CudaEngine : public Engine {
     int rc;
     if ((rc = upload(gb.probs, probs))) return rc;
     if ((rc = upload(gb.tiles, tiles))) return rc;
-    // FP64 batches run in 32 x 32 tiles while the device holds all of those
-    // at once (1480 on 148 SMs): 64 x 64 tiles then leave SMs idle or cover
-    // more padding.  Measured with k = 64, 128 and 256, the Schur scatter and
-    // square problems of 64 to 448 rows, 64 x 64 time / 32 x 32 time: up to
-    // 600 tiles of 32 1.4-2.0, up to 1480 1.04-1.9; from there to 1770, where
-    // a second wave begins while 64 x 64 tiles may still take one, 0.76-1.4;
-    // above that 0.94-1.7 as the 64 x 64 tiles' own waves fall.
+    // FP64 batches run in 32 x 32 tiles while the device takes at most two
+    // rounds of those (1480 tiles on 148 SMs): 64 x 64 tiles then leave SMs
+    // idle or cover more padding.  64 x 64 time / 32 x 32 time, measured with
+    // k = 64, 128 and 256, plain and scattering into parents, square problems
+    // of 64 to 448 rows: up to 600 tiles of 32 1.4-2.0, up to 1480 1.04-1.9;
+    // from there to 1770, a third round where 64 x 64 tiles may still take
+    // one, 0.76-1.4; above that 0.94-1.7.  On the batches of seven 2D and 3D
+    // grids: up to 1480 1.13-2.0, to 1770 0.96-1.09, to 6600 0.92-1.38, above
+    // that 0.85-1.1, the least where k is largest.
     int64_t n32 = 0;
     for (const GemmProb& g : probs)
       n32 += (int64_t)((g.m + 31) / 32) * ((g.n + 31) / 32);
@@ -3006,7 +3008,7 @@ class CudaEngine : public Engine {
   int force_tcp_ = -1;  // tensor-core kernel variant forced (-1: per batch)
   int force_width_ = -1;  // tensor-core tile width forced (0: 128, 1: 64)
   bool use_dmma_ = true;  // FP64 GEMMs on the FP64 tensor cores
-  int64_t dmma32_cap_ = 0;  // 32 x 32 tiles the device holds at once
+  int64_t dmma32_cap_ = 0;  // most 32 x 32 tiles of a batch that runs in them
   int force_split_ = -1;  // FP32 GEMM split for every batch: 0 TF32x3, 1 BF16x3
   bool deterministic_ = false;  // fixed-order reductions (SNU_DETERMINISTIC)
   int tcp_cap_[2] = {148, 148};  // persistent grid per tile width

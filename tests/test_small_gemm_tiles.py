@@ -1,5 +1,5 @@
-"""FP64 Schur updates of batches that the device holds at once in 32 x 32 tiles
-run in those: fronts whose update matrices end inside a tile, on one tile and
+"""FP64 Schur updates of batches of at most two rounds of 32 x 32 tiles run in
+those: fronts whose update matrices end inside a tile, on one tile and
 on several, and batches on both sides of that size, against the dense
 solution."""
 import numpy as np
@@ -39,7 +39,7 @@ def test_fp64_updates_on_both_sides_of_the_rule(gpu, copies, above):
         fp = s.front_plan()
         tiles = np.zeros(fp["nlevels"], int)  # 32 x 32 tiles of each level
         np.add.at(tiles, fp["level"], ((fp["q"] + 31) // 32) ** 2)
-        # (1480: ten blocks on each of 148 SMs)
+        # (1480: two rounds of five blocks on each of 148 SMs)
         assert tiles.max() > 1480 if above else tiles.max() <= 1480
         x = s.factorize().solve(b)
     for k in range(3):
