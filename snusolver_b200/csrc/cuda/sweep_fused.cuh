@@ -54,13 +54,15 @@ struct SweepDep {
 // off-diagonal tasks of f finished.
 __device__ __forceinline__ bool wait_count(const int* ctr, int target,
                                            int* err, long limit) {
-  for (long it = 0; it < limit; it++) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(ctr)
-                 : "memory");
-    if (v >= target) return true;
-    if (wait_failed(err, it)) break;
-    if (it > 4) __nanosleep(20);
+  for (long r = 0; r < limit; r += WAVE_ROUND) {
+    if (r > 0 && wait_failed(err)) break;
+    for (int it = 0; it < WAVE_ROUND; it++) {
+      int v;
+      asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(ctr)
+                   : "memory");
+      if (v >= target) return true;
+      if (it > 4) __nanosleep(20);
+    }
   }
   atomicExch(err, 1);
   return false;
