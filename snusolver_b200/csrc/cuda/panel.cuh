@@ -148,7 +148,7 @@ constexpr int SB = 4;  // pivots per step of the tile factorization
 // so every operand that several threads share is requested by as few of
 // them as possible: a chain of four warps beside update warps that also
 // collected took 1150 cycles a step where this takes 780.)  A full tile on
-// one SM takes 16.3 thousand cycles in FP32 and 28.3 in FP64, where the
+// one SM takes 16.3 thousand cycles in FP32 and 28.4 in FP64, where the
 // factorization by 16 x 16 sub-blocks with the inverses joined afterwards
 // took 21.5 and 44.7.
 //
@@ -260,10 +260,10 @@ __device__ __forceinline__ void diag_tile(const FrontDev& f,
     for (int s = 0; s < nsb; s++) {
       const int par = s & 1, s0 = SB * s;
       // the pivot block with the previous step's update.  FP32: every lane
-      // forms all of it.  FP64, where that is 64 multiply-adds at a sixteenth
-      // of a warp each: lane 4 a + c (and its copy 16 up) forms element
-      // (a, c) and all lanes gather the sixteen (28.4 against 30.1 thousand
-      // cycles a tile; FP32 16.5 against 15.8)
+      // forms all of it (gathering it as below costs 0.7 thousand cycles a
+      // tile).  FP64, where that is 64 multiply-adds at a sixteenth of a warp
+      // each: lane 4 a + c (and its copy 16 up) forms element (a, c) and all
+      // lanes gather the sixteen (28.4 against 30.1 thousand cycles a tile)
       T d[SB][SB], r[SB], xn[SB], yn[SB], e = (T)0;
       if constexpr (sizeof(T) == 8) {
         const int ea = (tid >> 2) & 3, ec = tid & 3;

@@ -26,8 +26,10 @@
 //   for the tile and forms U_t = Linv_t (A_t - sum_{s<t} L_ts U_s) for its
 //   columns (the U12 rows of the block, right of it).
 //
-// Four flags per tile s: [4 s] tile s factored (the tile, its inverses and
-// every L block of its rows stored), [4 s + 1] its owner's U rows right of
+// Four flags per tile s: [4 s] tile s factored (its inverses and every L block
+// of its rows stored; not the tile itself, which its owner stores after
+// raising the flag, as no other task of the launch reads it: whoever does
+// needs a flag of its own), [4 s + 1] its owner's U rows right of
 // the next tile stored, [4 s + 2] its U rows in the next tile's columns
 // stored (by the next tile's owner), [4 s + 3] the next tile's L block of
 // step s stored.  Every product is formed from the same operands in the
@@ -420,6 +422,10 @@ constexpr size_t block_smem() {
   return block_tiles<T>() * (size_t)tile_elems<T>() * sizeof(T);
 }
 
+// (Two CTAs an SM leave a thread 128 registers.  In FP64 the tile
+// factorization alone takes 138, so 148 bytes a thread are spilled; a tile
+// still takes 28.4 thousand cycles, where the sub-block form, which spilled
+// nothing, took 44.7.)
 template <typename T>
 __global__ void __launch_bounds__(256, 2)
     k_panel_block(const BlockTask* __restrict__ tasks, int ntasks,
@@ -492,7 +498,7 @@ __global__ void __launch_bounds__(256, 2)
             pb_load(S2, Fo + k0 + c0n * ld, ld, NB, ncn);
           }
         }
-                if (own) {
+        if (own) {
           // the diagonal tile (its columns are up to date; in S0 when our
           // work as the next owner left it there); Linv comes back in S1
           diag_tile<T>(f, F, INV, k0, step, eps, dflags, S0, S1,

@@ -16,8 +16,9 @@
 //
 // Each level of a sweep is two launches (more with work vectors):
 //
-// * the pivot block (rows and columns [0, p)): one cooperative launch over
-//   (front, 128-row chunk) tasks.  The chunk holding a tile's rows solves the
+// * the pivot block (rows and columns [0, p)): one launch over (front, 128-row
+//   chunk) tasks, taken from a counter (not a cooperative launch: it starts
+//   while the kernel before it runs).  The chunk holding a tile's rows solves the
 //   tile with the stored inverse of the diagonal tile and publishes the
 //   result in Y; the other chunks of the front wait for it (bounded spin) and
 //   update their rows.  Y itself is the flag: it starts as a NaN that no
@@ -266,11 +267,14 @@ __device__ __forceinline__ void lds(const T* p, T (&v)[N]) {
 // init(row, r): the chunk's starting right-hand side; done(row, r, v): what
 // else becomes of a solved element; Yp (columns ldy apart, column r0 first): where tiles are published and waited for.
 //
-// The chain of tiles is bound by the hand-over between CTAs and by shared
-// memory, which serves 128 requested bytes a cycle, broadcasts included.
+// The chain of tiles is bound by latency: its hand-overs between CTAs, and
+// shared-memory loads and barriers in front of few warps (one or two CTAs of
+// four warps an SM).  48^3 convection-diffusion, FP32, 64 columns (8): warps
+// active 6-12% (6-12), issue slots 20-42% (18-30), shared-memory wavefronts
+// 20-38% (22-31) of what the SM can serve, FMA pipe 12-26% (9-15).
 // So the chunk's right-hand side stays in registers, a thread holding TR rows
-// x TC columns (4 x 4 at 16 columns: 8 cycles of requests for 16
-// multiply-adds where a row per thread takes 17), and a tile is handed over
+// x TC columns (4 x 4 at 16 columns: two vector loads for 16 multiply-adds,
+// where a row per thread takes five), and a tile is handed over
 // through its values alone: no fence, flag or second load.  With the
 // products below, 64 columns on a 54^3 grid 20.1 -> 15.6 ms (pivot blocks
 // 9.5 -> 6.5, products 5.8 -> 3.9), 13 FP64 columns on 37^3 2.44 -> 1.66 ms.
@@ -585,10 +589,12 @@ constexpr int GEMV_ROWS = 64, GEMV_K = 256;
 // Blocks of one task are neighbours (they share its factor entries in L2)
 // and take columns [g R, g R + R) of the pass each.
 //
-// A lane holds two rows (one value of the vector slice, which shared memory
-// broadcasts at one requested word a cycle, serves two multiply-adds), a
-// warp an eighth of the columns; GEMV_LD of its factor entries are in
-// flight at a time, the first of them before the slice is staged.
+// A lane holds two rows (so a load of the vector slice serves two rows'
+// multiply-adds), a warp an eighth of the columns; UB columns of its factor
+// entries are in flight at a time, the first of them before the slice is
+// staged.  Bound by latency (48^3 convection-diffusion, FP32, 64 columns:
+// warps active 24%, issue slots 45-52%, shared-memory wavefronts 36-38%, FMA
+// pipe 25-30%; 8 columns: waiting on the factor loads).
 template <typename T, int R, bool FWD>
 __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
                                          int ngroups,

@@ -1,11 +1,10 @@
 // Dependency-driven triangular sweeps: the whole forward (or backward)
 // solve over the front tree in ONE cooperative launch.
 //
-// The level-by-level sweeps (sweep.cuh) take four launches per level and
-// direction (gathers, extend-adds, pivot blocks, off-diagonal products);
-// on the leaf levels, where fronts are small, those launches are mostly
-// latency.  Here every level's work is one task list and a front starts as
-// soon as what it reads is final:
+// The level-by-level sweeps (sweep.cuh) take two launches per level and
+// direction (pivot blocks, off-diagonal products); on the smallest trees
+// those launches are mostly latency.  Here every level's work is one task
+// list and a front starts as soon as what it reads is final:
 //
 // * forward: Z (elimination order, as in sweep.cuh) starts as B.  Pivot-block
 //   chunk task (f, c): waits until every off-diagonal task of f's children
