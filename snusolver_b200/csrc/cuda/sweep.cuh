@@ -270,8 +270,8 @@ __device__ __forceinline__ void lds(const T* p, T (&v)[N]) {
 // The chain of tiles is bound by latency: its hand-overs between CTAs, and
 // shared-memory loads and barriers in front of few warps (one or two CTAs of
 // four warps an SM).  48^3 convection-diffusion, FP32, 64 columns (8): warps
-// active 6-12% (6-12), issue slots 20-42% (18-30), shared-memory wavefronts
-// 20-38% (22-31) of what the SM can serve, FMA pipe 12-26% (9-15).
+// active 6-12% (6-12), issue slots 23-44% (21-32), shared-memory wavefronts
+// 20-39% (20-34) of what the SM can serve, FMA pipe 13-28% (10-16).
 // So the chunk's right-hand side stays in registers, a thread holding TR rows
 // x TC columns (4 x 4 at 16 columns: two vector loads for 16 multiply-adds,
 // where a row per thread takes five), and a tile is handed over
@@ -593,8 +593,8 @@ constexpr int GEMV_ROWS = 64, GEMV_K = 256;
 // multiply-adds), a warp an eighth of the columns; UB columns of its factor
 // entries are in flight at a time, the first of them before the slice is
 // staged.  Bound by latency (48^3 convection-diffusion, FP32, 64 columns:
-// warps active 24%, issue slots 45-52%, shared-memory wavefronts 36-38%, FMA
-// pipe 25-30%; 8 columns: waiting on the factor loads).
+// warps active 24%, issue slots 45-52%, shared-memory wavefronts 34-39%, FMA
+// pipe 26-29%; 8 columns: waiting on the factor loads).
 template <typename T, int R, bool FWD>
 __device__ __forceinline__ void gemv_off(const SweepTask* __restrict__ tasks,
                                          int ngroups,
